@@ -250,12 +250,13 @@ static int build_mesh(ccs_handle *h, const ccs_mesh_view *mv) {
   const Layout &L = h->L;
   const size_t nref = (size_t)L.nh * L.nh * 6;
   const size_t nf = (size_t)L.field;
-  // 15 FP64 arrays: sqrtG phis f ig11 ig12 ig21 ig22 aig11..22 gia11..22
-  CCS_TRY(h, cudaMalloc(&dm->buf64, 15 * nf * sizeof(double)));
-  CCS_TRY(h, cudaMemsetAsync(dm->buf64, 0, 15 * nf * sizeof(double), h->stream));
-  std::vector<double> tmp(15 * nref, 0.);
-  double *t[15];
-  for (int k = 0; k < 15; k++) t[k] = tmp.data() + k * nref;
+  // FP64 arrays: sqrtG phis f ig11 ig12 ig21 ig22 aig11..22 gia11..22 sqrtGf rsqrtG lamx lamy
+  constexpr int na = 19;
+  CCS_TRY(h, cudaMalloc(&dm->buf64, na * nf * sizeof(double)));
+  CCS_TRY(h, cudaMemsetAsync(dm->buf64, 0, na * nf * sizeof(double), h->stream));
+  std::vector<double> tmp(na * nref, 0.);
+  double *t[na];
+  for (int k = 0; k < na; k++) t[k] = tmp.data() + k * nref;
   for (size_t c = 0; c < nref; c++) {
     t[0][c] = mv->sqrtG[c];
     t[1][c] = mv->phis[c];
@@ -270,8 +271,18 @@ static int build_mesh(ccs_handle *h, const ccs_mesh_view *mv) {
     t[7][c] = M[0]; t[8][c] = M[2]; t[9][c] = M[1]; t[10][c] = M[3];
     matmul22(&mv->matrixG[4 * c], &mv->matrixIA[4 * c], M);  // projection_mod.F90:71
     t[11][c] = M[0]; t[12][c] = M[2]; t[13][c] = M[1]; t[14][c] = M[3];
+    t[15][c] = mv->sqrtG[c] * mv->f[c];
+    t[16][c] = 1. / mv->sqrtG[c];
   }
-  for (int k = 0; k < 15; k++) {
+  const size_t nh = L.nh;
+  for (int p = 0; p < 6; p++)  // face means (spatial_operators_mod.F90:113-114, 138-139)
+    for (size_t j = 0; j < nh; j++)
+      for (size_t i = 0; i < nh; i++) {
+        const size_t c = i + nh * (j + nh * p);
+        if (i + 1 < nh) t[17][c] = 0.5 * (mv->matrixIG[4 * (c + 1)] + mv->matrixIG[4 * c]);
+        if (j + 1 < nh) t[18][c] = 0.5 * (mv->matrixIG[4 * (c + nh) + 3] + mv->matrixIG[4 * c + 3]);
+      }
+  for (int k = 0; k < na; k++) {
     int rc = upload_field(h, dm->buf64 + k * nf, t[k]);
     if (rc) return rc;
   }
@@ -280,6 +291,7 @@ static int build_mesh(ccs_handle *h, const ccs_mesh_view *mv) {
   dm->m64.ig11 = b + 3 * nf; dm->m64.ig12 = b + 4 * nf; dm->m64.ig21 = b + 5 * nf; dm->m64.ig22 = b + 6 * nf;
   dm->m64.aig11 = b + 7 * nf; dm->m64.aig12 = b + 8 * nf; dm->m64.aig21 = b + 9 * nf; dm->m64.aig22 = b + 10 * nf;
   dm->m64.gia11 = b + 11 * nf; dm->m64.gia12 = b + 12 * nf; dm->m64.gia21 = b + 13 * nf; dm->m64.gia22 = b + 14 * nf;
+  dm->m64.sqrtGf = b + 15 * nf; dm->m64.rsqrtG = b + 16 * nf; dm->m64.lamx = b + 17 * nf; dm->m64.lamy = b + 18 * nf;
   std::vector<int32_t> push;
   if (!build_push_table(L, push)) {
     h->err = "ghost tables are inconsistent";

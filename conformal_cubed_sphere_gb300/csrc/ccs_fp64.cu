@@ -3,7 +3,12 @@
 // Built with -fmad=false: every operation below is a separately rounded IEEE
 // double operation in the order of the Fortran source (left to right), so the
 // result is bitwise the reference arithmetic (gfortran -fdefault-real-8 on x86-64
-// emits no FMA).  `/` and sqrt are the IEEE-rounded CUDA double operations.
+// emits no FMA).
+//
+// Bound: the FP64 pipe, two lanes per SM and cycle.  So the reconstructions take what
+// depends on one cell or one second difference from shared memory, where each is
+// formed once, and their quotients run on the integer pipes (ccs_softfp.cuh): FP64
+// instructions per cell and stage 1878 -> 607, C384 stage 3160 -> 1219 us.
 //
 // A CTA owns a tile of F64_TX x F64_TY interior cells of one panel.  It stages the
 // halo'd tile (3 cells each side) of the cell quantities of the spatial operator
@@ -19,10 +24,14 @@
 // stage is the whole grid-wide dependency.
 #include "ccs_kernels.h"
 #include "ccs_bounds.cuh"
+#include "ccs_softfp.cuh"
 
 namespace ccs {
 
 namespace {
+
+// arrays of single-cell products of a reconstructed field (see side)
+constexpr int NSING = 6;
 
 // a tile of TX x TY cells; phase 3 maps one thread to one cell
 template <int TX_, int TY_>
@@ -30,9 +39,12 @@ struct F64Tile {
   static constexpr int TX = TX_, TY = TY_, NT = TX * TY;
   static constexpr int RX = TX + 6, RY = TY + 6, RN = RX * RY;
   static constexpr int NFX = TY * (TX + 1), NFY = (TY + 1) * TX, NF = NFX + NFY;
+  // cells of the lines through the tile: rows of RX cells, columns of RY
+  static constexpr int NLX = TY * RX, NLY = RY * TX;
+  static constexpr int NSCR_F = (NSING + 2) * (NLX + NLY), NSCR_E = NSING * RN + 2 * (NLX + NLY);
+  static constexpr int NSCR = NSCR_F > NSCR_E ? NSCR_F : NSCR_E;
 };
 constexpr int NT = 256;
-constexpr int NCELL_ARR = 11;
 
 }  // namespace
 
@@ -65,6 +77,14 @@ __device__ __forceinline__ double ccs_div_by(double a, double b, double y) {
   const double q0 = a * y;
   const double r = fma(-q0, b, a);
   return fma(r, y, q0);
+}
+
+// phiG / sqrtG from the grid's reciprocals y = RN(1 / sqrtG); a phiG so small that the
+// quotient might not be normal takes IEEE division
+__device__ __forceinline__ double div_depth(double x, double b, double y) {
+  const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+  if (e < 257u && x != 0.) return x / b;
+  return ccs_div_const(x, b, y);
 }
 
 namespace {
@@ -149,14 +169,208 @@ __device__ __forceinline__ double central_diff(int op, const double *f, int s, d
   return (-f[-3 * s] + 9. * f[-2 * s] - 45. * f[-s] + 45. * f[s] - 9. * f[2 * s] + f[3 * s]) / (60. * d);
 }
 
-template <int RN>
+// x / 2 of a normal x by its exponent; zeros, infinities, NaNs and values at the
+// bottom of the range take the FP64 multiplication
+__device__ __forceinline__ double half_of(double x) {
+  const uint32_t h = softfp::hi32(softfp::bits_of(x)), e = h & 0x7ff00000u;
+  if (e - 0x00200000u < 0x7fc00000u) return __hiloint2double((int)(h - 0x00100000u), __double2loint(x));
+  return 0.5 * x;
+}
+
+// Whether the integer arithmetic of the reconstructions covers a field value: zero or
+// of magnitude in [2^-200, 2^200).  Differences of such values are zero or at least
+// 2^-253, so the smoothness indicators lie in {0} or [2^-510, 2^410], the weights in
+// [2^-415, 1], and no product, sum or quotient of a reconstruction leaves the normal range.
+__device__ __forceinline__ bool in_window(double x) {
+  const unsigned long long t = (unsigned long long)__double_as_longlong(x) << 1;
+  return t == 0ull || t - ((unsigned long long)(1023 - 200) << 53) < ((unsigned long long)400 << 53);
+}
+
+// One WENO-Z reconstruction (WENO_limiter, spatial_operators_mod.F90:282-361) of a
+// cell's value at one of its two faces, in the reference's order of operations:
+// Q at stride +s for the "+" side (face after the cell), -s for the "-" side, whose
+// formulas are the mirrored ones.  What depends on a single cell, or on three cells
+// alike in the neighbouring reconstructions, comes from shared memory:
+//   G[0..5] at the cell, arrays SG apart: Q/3, 7/6 Q, 11/6 Q, 5/6 Q, 1/3 Q, 3 Q
+//   ga at the cell: 13/12 (second difference centred there)^2, same orientation
+// (Q/6 and 1/6 Q are exact halves of Q/3 and 1/3 Q; multiplications by 2, 4 and 1/4 are
+// exact and fuse.)  The quotients run on the integer pipes (ccs_softfp.cuh).
+__device__ __forceinline__ double side(const double *Q, int s, const double *G, int SG, int gs, const double *ga,
+                                       int as) {
+  const double q3 = G[5 * SG];
+  const double b0 = fma(-4., Q[-s], Q[-2 * s]) + q3;
+  const double b1 = Q[-s] - Q[s];
+  const double b2 = fma(-4., Q[s], q3) + Q[2 * s];
+  const double be0 = fma(b0 * b0, 0.25, ga[-as]);
+  const double be1 = fma(b1 * b1, 0.25, ga[0]);
+  const double be2 = fma(b2 * b2, 0.25, ga[as]);
+  // the betas are sums of squares (never -0 or negative), the taus absolute values
+  const long long t40 = abs_bits(be0 - be1), t41 = abs_bits(be1 - be2);
+  const double tau5 = fabs(be2 - be0);
+  long long mn = __double_as_longlong(be0);
+  if (__double_as_longlong(be1) < mn) mn = __double_as_longlong(be1);
+  if (__double_as_longlong(be2) < mn) mn = __double_as_longlong(be2);
+  double w0, w1, w2;
+  if (t40 <= mn && t41 > mn) {
+    w0 = 1. / 3.; w1 = 2. / 3.; w2 = 0.;
+  } else if (t40 > mn && t41 < mn) {
+    w0 = 0.; w1 = 2. / 3.; w2 = 1. / 3.;
+  } else {
+    using namespace softfp;
+    const double eps = 1.E-2;
+    const Unp k01{0xccccccccccccd000ull, 1019}, k06{0x9999999999999800ull, 1022}, k03{0x9999999999999800ull, 1021};
+    const Unp t = unpack(tau5);  // tau5 = 0 reads as 2^-1023: 1 + tau5 / .. rounds to 1 either way
+    const Unp p0 = one_plus(div(t, divisor(unpack(eps + be0))));
+    const Unp p1 = one_plus(div(t, divisor(unpack(eps + be1))));
+    const Unp p2 = one_plus(div(t, divisor(unpack(eps + be2))));
+    const Unp a0 = mul(p0, k01), a1 = mul(p1, k06), a2 = mul(p2, k03);
+    const Divisor d = divisor(unpack((pack(a0) + pack(a1)) + pack(a2)));
+    w0 = pack(div(a0, d));
+    w1 = pack(div(a1, d));
+    w2 = pack(div(a2, d));
+  }
+  const double s0 = (G[-2 * gs] - G[SG - gs]) + G[2 * SG];
+  const double s1 = fma(-0.5, G[-gs], G[3 * SG]) + G[4 * SG + gs];
+  const double s2 = fma(-0.5, G[4 * SG + 2 * gs], G[0] + G[3 * SG + gs]);
+  return fma(s0, w0, 0.) + s1 * w1 + s2 * w2;
+}
+
+// 13/12 a^2 rounded as the reference does: ((a a) 13) / 12
+__device__ __forceinline__ double curvature(double a) {
+  using namespace softfp;
+  const Unp u = unpack(a);
+  Unp g = div3(mul13(mul(u, u)));
+  g.e -= 2;
+  return a == 0. ? 0. : pack(g);
+}
+
+template <class T>
 struct Smem {
   // cell quantities on the halo'd tile (row-major [RY][RX])
-  double phit[RN], phitG[RN], E[RN], Fx[RN], Fy[RN], uC[RN], vC[RN], ig11[RN], ig22[RN], u[RN], v[RN];
+  double phit[T::RN], phitG[T::RN], E[T::RN], Fx[T::RN], Fy[T::RN], uC[T::RN], vC[T::RN], u[T::RN], v[T::RN];
+  // face values: sums of the two sides of the flux and E, difference of phitG's (and of
+  // the wind's: E dissipation); then the Rusanov fluxes of phiG and E in the first two
+  double rec[4][T::NF];
+  // per-cell products of the fields of one pass: either fields of their own on the rows
+  // and columns, or one field on the halo'd tile with curvatures on rows and columns
+  double scr[T::NSCR];
 };
 
 __device__ __forceinline__ bool is_corner(int i, int j, int N) {
   return (i < 1 || i > N) && (j < 1 || j > N);
+}
+
+__device__ __forceinline__ void store_singles(double *G, int SG, double q) {
+  using namespace softfp;
+  const Unp t = div3(unpack(q));
+  const double third = __longlong_as_double(
+      q == 0. ? __double_as_longlong(q)
+              : __double_as_longlong(pack(t)) | (__double_as_longlong(q) & (long long)0x8000000000000000ull));
+  G[0] = third;
+  G[SG] = 7. / 6. * q;
+  G[2 * SG] = 11. / 6. * q;
+  G[3 * SG] = 5. / 6. * q;
+  G[4 * SG] = 1. / 3. * q;
+  G[5 * SG] = fma(2., q, q);
+}
+
+// Reconstructs one pass of fields at every face of the tile, both sides: QX along the
+// rows and QY along the columns (the same array for E and phitG).  rec receives
+// (+) + (-) or, with DIFF, (-) - (+).  nx, ny: the tile's cells inside the panel.
+template <class T, bool SAME, bool DIFF>
+__device__ __forceinline__ void reconstruct(Smem<T> &S, const double *QX, const double *QY, double *rec, int nx,
+                                            int ny, bool slow) {
+  constexpr int TX = T::TX, TY = T::TY, RX = T::RX, RY = T::RY, RN = T::RN, NLX = T::NLX, NLY = T::NLY;
+  constexpr int NFX = T::NFX, NF = T::NF;
+  const int tid = threadIdx.x;
+  // products: [NSING] arrays on the halo'd tile (SAME) or on the rows / columns, then
+  // the curvatures of the "+" and "-" orientation on the rows and on the columns
+  double *GX = S.scr, *GY = SAME ? S.scr : S.scr + NSING * NLX;
+  constexpr int SGX = SAME ? RN : NLX, SGY = SAME ? RN : NLY;
+  double *AX = S.scr + (SAME ? NSING * RN : NSING * (NLX + NLY)), *AY = AX + 2 * NLX;
+  if (!slow) {
+    if constexpr (SAME) {
+      for (int r = tid; r < RN; r += NT) store_singles(GX + r, SGX, QX[r]);
+    } else {
+      for (int r = tid; r < NLX + NLY; r += NT) {
+        if (r < NLX) {
+          store_singles(GX + r, SGX, QX[3 * RX + r]);
+        } else {
+          const int q = r - NLX;
+          store_singles(GY + q, SGY, QY[(q / TX) * RX + q % TX + 3]);
+        }
+      }
+    }
+    for (int r = tid; r < 2 * (NLX + NLY); r += NT) {
+      const bool minus = r >= NLX + NLY;
+      const int q = minus ? r - (NLX + NLY) : r;
+      const double *f;
+      double *o;
+      int st;
+      bool in;
+      if (q < NLX) {
+        const int ci = q % RX;
+        in = ci >= 1 && ci < RX - 1;
+        f = QX + 3 * RX + q;
+        st = 1;
+        o = AX + (minus ? NLX : 0) + q;
+      } else {
+        const int k = q - NLX, cj = k / TX;
+        in = cj >= 1 && cj < RY - 1;
+        f = QY + cj * RX + k % TX + 3;
+        st = RX;
+        o = AY + (minus ? NLY : 0) + k;
+      }
+      if (in) {
+        const int d = minus ? -st : st;
+        *o = curvature(fma(-2., f[0], f[-d]) + f[d]);
+      }
+    }
+    __syncthreads();
+  }
+  // lanes 2 k and 2 k + 1 take the two sides of one face
+  for (int t0 = tid & ~31; t0 < 2 * NF; t0 += NT) {
+    const int t = t0 + (tid & 31), face = t >> 1, minus = t & 1;
+    double val = 0.;
+    if (t < 2 * NF) {
+      bool in;
+      int cell, lcell, st, ls;  // the cell in the halo'd tile and on its line's arrays
+      const double *f;
+      const double *G, *A;
+      if (face < NFX) {
+        const int lj = face / (TX + 1), ci = face % (TX + 1) + 2 + minus;
+        in = lj < ny && ci - 2 - minus <= nx;
+        cell = (lj + 3) * RX + ci;
+        lcell = lj * RX + ci;
+        st = ls = 1;
+        f = QX;
+        G = GX + (SAME ? cell : lcell);
+        A = AX + (minus ? NLX : 0);
+      } else {
+        const int fy = face - NFX, li = fy % TX, cj = fy / TX + 2 + minus;
+        in = li < nx && cj - 2 - minus <= ny;
+        cell = cj * RX + li + 3;
+        lcell = cj * TX + li;
+        st = RX;
+        ls = TX;
+        f = QY;
+        G = GY + (SAME ? cell : lcell);
+        A = AY + (minus ? NLY : 0);
+      }
+      if (in && ccs_inb(cell - 2 * st, RN, 211) && ccs_inb(cell + 2 * st, RN, 212)) {
+        f += cell;
+        if (minus) { st = -st; ls = -ls; }
+        if (slow)
+          val = minus ? weno5z<-1>(f[2 * st], f[st], f[0], f[-st], f[-2 * st])
+                      : weno5z<1>(f[-2 * st], f[-st], f[0], f[st], f[2 * st]);
+        else
+          val = side(f, st, G, face < NFX ? SGX : SGY, SAME ? st : ls, A + lcell, ls);
+      }
+    }
+    const double other = __shfl_xor_sync(0xffffffffu, val, 1);
+    if (!minus && t < 2 * NF && ccs_inb(face, NF, 213)) rec[face] = DIFF ? other - val : val + other;
+  }
+  __syncthreads();
 }
 
 template <class T>
@@ -165,8 +379,7 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
   constexpr int TX = T::TX, TY = T::TY, RX = T::RX, RN = T::RN, NFX = T::NFX, NF = T::NF;
   static_assert(T::NT == NT, "phase 3 maps one thread to one cell");
   extern __shared__ __align__(16) double smem_raw[];
-  Smem<RN> &S = *reinterpret_cast<Smem<RN> *>(smem_raw);
-  double *rec = smem_raw + NCELL_ARR * RN;  // [nrec][NF]
+  Smem<T> &S = *reinterpret_cast<Smem<T> *>(smem_raw);
   const int tid = threadIdx.x;
 
   for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
@@ -175,21 +388,24 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
     const Layout L = st.L;
     const int N = L.N, p = wi.panel;
     const int i0 = 1 + wi.tx * TX, j0 = 1 + wi.ty * TY;
-    const int nrec = st.ediss ? 8 : 6;
+    const bool ediss = st.ediss != 0;
     const int op = st.op;  // uniform over the work item
 #ifdef CCS_BOUNDS
     // poison the tile arrays: a read of a slot this tile never wrote shows up as NaN
     // in the result (checked build only)
-    for (int k = tid; k < NCELL_ARR * RN + 8 * NF; k += NT) smem_raw[k] = __longlong_as_double(0x7ff8000000000000LL);
+    for (int k = tid; k < (int)(sizeof(S) / sizeof(double)); k += NT)
+      smem_raw[k] = __longlong_as_double(0x7ff8000000000000LL);
     __syncthreads();
 #endif
 
     // ---- phase 1: cell quantities (spatial_operators_mod.F90:71-78) ----------
+    // (cells outside the panel and its edge halos are set to zero: the faces that
+    // would read them belong to no interior cell)
+    bool odd = false;
     for (int r = tid; r < RN; r += NT) {
       const int li = r % RX, lj = r / RX;
       const int i = i0 - 3 + li, j = j0 - 3 + lj;
-      double phit = 0., phitG = 0., E = 0., Fx = 0., Fy = 0., uC = 0., vC = 0., g11 = 0., g22 = 0., u = 0.,
-             v = 0.;
+      double phit = 0., phitG = 0., E = 0., Fx = 0., Fy = 0., uC = 0., vC = 0., u = 0., v = 0.;
       const int64_t c = L.idx(i, j, p);
       if (i >= -2 && i <= N + 3 && j >= -2 && j <= N + 3 && !is_corner(i, j, N) && ccs_inb(c, L.field, 201)) {
         const double phiG = st.in.phiG[c], phi = st.in.phi[c];
@@ -197,91 +413,66 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
         v = st.in.v[c];
         uC = st.in.uC[c];
         vC = st.in.vC[c];
-        g11 = st.m.ig11[c];
-        g22 = st.m.ig22[c];
         phit = phi + st.m.phis[c];
         phitG = phit * st.m.sqrtG[c];
-        const double K = 0.5 * (u * uC + v * vC);
+        const double K = half_of(u * uC + v * vC);
         E = phit + K;
         Fx = phiG * uC;
         Fy = phiG * vC;
+        odd = odd || __double_as_longlong(phit) <= 0 || !in_window(phitG) || !in_window(E) || !in_window(Fx) || !in_window(Fy) ||
+              !in_window(u) || !in_window(v);
       }
       S.phit[r] = phit; S.phitG[r] = phitG; S.E[r] = E; S.Fx[r] = Fx; S.Fy[r] = Fy;
-      S.uC[r] = uC; S.vC[r] = vC; S.ig11[r] = g11; S.ig22[r] = g22; S.u[r] = u; S.v[r] = v;
+      S.uC[r] = uC; S.vC[r] = vC; S.u[r] = u; S.v[r] = v;
     }
-    __syncthreads();
+    // a tile with values outside the window of the integer arithmetic (or without
+    // positive depth) takes the FP64 instructions throughout
+    const bool slow = __syncthreads_or(odd);
+    const int nx = min(TX, N + 1 - i0), ny = min(TY, N + 1 - j0);
 
     // ---- phase 2: face reconstructions (weno, :183-277) ---------------------
     // (the central-difference operators have no faces: straight to phase 3)
     if (op == CCS_OP_WENO) {
-    for (int t = tid; t < nrec * NF; t += NT) {
-      const int face = t % NF, q = t / NF;
-      const double *fld;
-      double val = 0.;
-      if (face < NFX) {
-        const int fi = face % (TX + 1), lj = face / (TX + 1);
-        const int f = i0 - 1 + fi, j = j0 + lj;
-        if (j <= N && f <= N && ccs_inb((lj + 3) * RX + fi + 5, RN, 211)) {
-          fld = (q < 2) ? S.Fx : (q < 4) ? S.E : (q < 6) ? S.phitG : S.u;
-          const double *row = fld + (lj + 3) * RX;
-          if ((q & 1) == 0)  // "+" from cell f: field(f-2 .. f+2)
-            val = weno5z<1>(row[fi], row[fi + 1], row[fi + 2], row[fi + 3], row[fi + 4]);
-          else  // "-" from cell f+1: field(f-1 .. f+3)
-            val = weno5z<-1>(row[fi + 1], row[fi + 2], row[fi + 3], row[fi + 4], row[fi + 5]);
-        }
-      } else {
-        const int fy = face - NFX;
-        const int li = fy % TX, fj = fy / TX;
-        const int g = j0 - 1 + fj, i = i0 + li;
-        if (i <= N && g <= N && ccs_inb(li + 3 + (fj + 5) * RX, RN, 212)) {
-          fld = (q < 2) ? S.Fy : (q < 4) ? S.E : (q < 6) ? S.phitG : S.v;
-          const double *col = fld + (li + 3);
-          if ((q & 1) == 0)
-            val = weno5z<1>(col[fj * RX], col[(fj + 1) * RX], col[(fj + 2) * RX], col[(fj + 3) * RX],
-                            col[(fj + 4) * RX]);
-          else
-            val = weno5z<-1>(col[(fj + 1) * RX], col[(fj + 2) * RX], col[(fj + 3) * RX], col[(fj + 4) * RX],
-                             col[(fj + 5) * RX]);
-        }
-      }
-      if (ccs_inb(q * NF + face, 8 * NF, 213)) rec[q * NF + face] = val;
-    }
-    __syncthreads();
+    reconstruct<T, false, false>(S, S.Fx, S.Fy, S.rec[0], nx, ny, slow);
+    reconstruct<T, true, false>(S, S.E, S.E, S.rec[1], nx, ny, slow);
+    reconstruct<T, true, true>(S, S.phitG, S.phitG, S.rec[2], nx, ny, slow);
+    if (ediss) reconstruct<T, false, true>(S, S.u, S.v, S.rec[3], nx, ny, slow);
 
     // ---- phase 2b: Rusanov fluxes at faces (:101-149) ------------------------
     for (int face = tid; face < NF; face += NT) {
-      const double Fp = rec[0 * NF + face], Fn = rec[1 * NF + face];
-      const double Ep = rec[2 * NF + face], En = rec[3 * NF + face];
-      const double Pp = rec[4 * NF + face], Pn = rec[5 * NF + face];
-      double dp = 0., dn = 0.;  // never-written u_ext / v_ext slots (CCS_EDISS_ZERO)
-      if (nrec == 8) {
-        dp = rec[6 * NF + face];
-        dn = rec[7 * NF + face];
-      }
-      double a, b, ga, gb, pa, pb;  // contravariant wind, IG diagonal, phit at the two cells
+      double a, b, pa, pb, lam;  // contravariant wind and phit at the two cells, mean IG diagonal
       if (face < NFX) {
         const int fi = face % (TX + 1), lj = face / (TX + 1);
         const int r = (lj + 3) * RX + fi + 2;  // cell f; cell f+1 is r + 1
-        if (!ccs_inb(r + 1, RN, 214)) continue;
+        if (i0 - 1 + fi > N || j0 + lj > N || !ccs_inb(r + 1, RN, 214)) continue;
         a = S.uC[r + 1]; b = S.uC[r];
-        ga = S.ig11[r + 1]; gb = S.ig11[r];
         pa = S.phit[r + 1]; pb = S.phit[r];
+        lam = st.m.lamx[L.idx(i0 - 1 + fi, j0 + lj, p)];
       } else {
         const int fy = face - NFX;
         const int li = fy % TX, fj = fy / TX;
         const int r = (fj + 2) * RX + li + 3;  // cell g; cell g+1 is r + RX
-        if (!ccs_inb(r + RX, RN, 215)) continue;
+        if (i0 + li > N || j0 - 1 + fj > N || !ccs_inb(r + RX, RN, 215)) continue;
         a = S.vC[r + RX]; b = S.vC[r];
-        ga = S.ig22[r + RX]; gb = S.ig22[r];
         pa = S.phit[r + RX]; pb = S.phit[r];
+        lam = st.m.lamy[L.idx(i0 + li, j0 - 1 + fj, p)];
       }
-      const double uBdy = 0.5 * (a + b);
-      const double phitBdy = 0.5 * (pa + pb);
-      const double e1 = uBdy - sqrt(0.5 * (ga + gb) * phitBdy);
-      const double e2 = uBdy + sqrt(0.5 * (ga + gb) * phitBdy);
-      const double mx = abs_bits(e2) > abs_bits(e1) ? fabs(e2) : fabs(e1);
-      rec[0 * NF + face] = 0.5 * (Fp + Fn - mx * (Pn - Pp));
-      rec[1 * NF + face] = 0.5 * (Ep + En - mx * (dn - dp));
+      const double uBdy = half_of(a + b);
+      const double phitBdy = half_of(pa + pb);
+      // max(|u - c|, |u + c|) = |u| + c, rounded alike
+      const double cs = sqrt(lam * phitBdy);
+      double mx = fabs(uBdy) + cs;
+      if (slow) {  // (a cell that is not finite keeps the reference's comparison)
+        const double e1 = uBdy - cs, e2 = uBdy + cs;
+        mx = abs_bits(e2) > abs_bits(e1) ? fabs(e2) : fabs(e1);
+      }
+      const double FS = S.rec[0][face], PD = S.rec[2][face];
+      double ES = S.rec[1][face];
+      // the never-written u_ext / v_ext slots (CCS_EDISS_ZERO) contribute mx (0 - 0): zero
+      // but for a wave speed that is not finite
+      if (ediss || slow) ES = ES - mx * (ediss ? S.rec[3][face] : 0.);
+      S.rec[0][face] = half_of(FS - mx * PD);
+      S.rec[1][face] = half_of(ES);
     }
     __syncthreads();
     }  // op == CCS_OP_WENO
@@ -296,7 +487,7 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
           ccs_inb(NFX + (lj + 1) * TX + li, NF, 223)) {
         double dfluxdx, dEdx, dvdx, dfluxdy, dEdy, dudy;
         if (op == CCS_OP_WENO) {
-          const double *FF = rec, *EF = rec + NF;
+          const double *FF = S.rec[0], *EF = S.rec[1];
           const int xl = lj * (TX + 1) + li, xr = xl + 1;
           const int yb = NFX + lj * TX + li, yt = yb + TX;
           // divisions by dx, dy, 60 dx, 60 dy (spatial_operators_mod.F90:153-169) from
@@ -320,8 +511,7 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
           dEdy = central_diff(op, S.E + rc, RX, st.dy);
           dudy = central_diff(op, S.u + rc, RX, st.dy);
         }
-        const double sqrtG = st.m.sqrtG[c];
-        const double vort = dvdx - dudy + sqrtG * st.m.f[c];
+        const double vort = dvdx - dudy + st.m.sqrtGf[c];
         const double uCc = S.uC[rc], vCc = S.vC[rc];
         const double tp = -(dfluxdx + dfluxdy);
         const double tu = -dEdx + vort * vCc;
@@ -340,9 +530,9 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
               np = y0p + st.c1 * tp; nu = y0u + st.c1 * tu; nv = y0v + st.c1 * tv;
               break;
             case K_RK4_2: {
-              const double ap = st.accphiG[c] + 2. * tp;
-              const double au = st.accu[c] + 2. * tu;
-              const double av = st.accv[c] + 2. * tv;
+              const double ap = fma(2., tp, st.accphiG[c]);
+              const double au = fma(2., tu, st.accu[c]);
+              const double av = fma(2., tv, st.accv[c]);
               st.accphiG[c] = ap; st.accu[c] = au; st.accv[c] = av;
               np = y0p + st.c1 * tp; nu = y0u + st.c1 * tu; nv = y0v + st.c1 * tv;
               break;
@@ -382,7 +572,7 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
           st.out.v[c] = v2;
           st.out.uC[c] = st.m.ig11[c] * u2 + st.m.ig12[c] * v2;
           st.out.vC[c] = st.m.ig21[c] * u2 + st.m.ig22[c] * v2;
-          st.out.phi[c] = np / sqrtG;
+          st.out.phi[c] = div_depth(np, st.m.sqrtG[c], st.m.rsqrtG[c]);
           if (st.zonal) {
             st.zonal[c] = zon;
             st.merid[c] = mer;
@@ -408,7 +598,7 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
             st.out.v[d] = vd;
             st.out.uC[d] = st.m.ig11[d] * ud + st.m.ig12[d] * vd;
             st.out.vC[d] = st.m.ig21[d] * ud + st.m.ig22[d] * vd;
-            st.out.phi[d] = np / st.m.sqrtG[d];
+            st.out.phi[d] = div_depth(np, st.m.sqrtG[d], st.m.rsqrtG[d]);
             if (st.zonal) {
               st.zonal[d] = zon;
               st.merid[d] = mer;
@@ -460,8 +650,8 @@ using F64T1 = F64Tile<16, 16>;
 using F64T2 = F64Tile<64, 4>;
 
 template <class T>
-constexpr int f64_smem_bytes() {  // sized for the E-reconstruction variant (8 face arrays)
-  return (int)((NCELL_ARR * T::RN + 8 * T::NF) * sizeof(double));
+constexpr int f64_smem_bytes() {
+  return (int)sizeof(Smem<T>);
 }
 
 template <class T>
