@@ -5,10 +5,15 @@
 // result is bitwise the reference arithmetic (gfortran -fdefault-real-8 on x86-64
 // emits no FMA).
 //
-// Bound: the FP64 pipe, two lanes per SM and cycle.  So the reconstructions take what
-// depends on one cell or one second difference from shared memory, where each is
-// formed once, and their quotients run on the integer pipes (ccs_softfp.cuh): FP64
-// instructions per cell and stage 1878 -> 607, C384 stage 3160 -> 1219 us.
+// Bound: the FP64 pipe, two lanes per SM and cycle (about 80 % busy at C384).  So the
+// reconstructions take what depends on one cell or one second difference from shared
+// memory, where each is formed once; quotients, square roots, the alphas of the WENO-Z
+// weights and the constant multiples of cell values run on the integer pipes
+// (ccs_softfp.cuh), which also round like IEEE; what stays is written as FMAs (F64Ops).
+// C384 stage with 16 x 16 tiles: 3160 us with every operation on the FP64 pipe, 1219 with
+// shared products and integer quotients, 946 now; FP64 thread instructions per cell and
+// stage 1780 -> 490.  Products of two variables (squares, weight times stencil) are no
+// faster in integers (+2 %) and stay.
 //
 // A CTA owns a tile of F64_TX x F64_TY interior cells of one panel.  It stages the
 // halo'd tile (3 cells each side) of the cell quantities of the spatial operator
@@ -36,7 +41,7 @@ constexpr int NSING = 6;
 // a tile of TX x TY cells; phase 3 maps one thread to one cell
 template <int TX_, int TY_>
 struct F64Tile {
-  static constexpr int TX = TX_, TY = TY_, NT = TX * TY;
+  static constexpr int TX = TX_, TY = TY_, NC = TX * TY;
   static constexpr int RX = TX + 6, RY = TY + 6, RN = RX * RY;
   static constexpr int NFX = TY * (TX + 1), NFY = (TY + 1) * TX, NF = NFX + NFY;
   // cells of the lines through the tile: rows of RX cells, columns of RY
@@ -44,7 +49,10 @@ struct F64Tile {
   static constexpr int NSCR_F = (NSING + 2) * (NLX + NLY), NSCR_E = NSING * RN + 2 * (NLX + NLY);
   static constexpr int NSCR = NSCR_F > NSCR_E ? NSCR_F : NSCR_E;
 };
-constexpr int NT = 256;
+// 12 warps and two CTAs an SM (80 registers): the FP64 pipe is shared by the whole SM,
+// and a warp holds it for a fraction of its time (C384 stage: 8 warps 1023 us, 12 warps
+// 989, 16 warps, which spill, 1032)
+constexpr int NT = 384;
 
 }  // namespace
 
@@ -77,14 +85,6 @@ __device__ __forceinline__ double ccs_div_by(double a, double b, double y) {
   const double q0 = a * y;
   const double r = fma(-q0, b, a);
   return fma(r, y, q0);
-}
-
-// phiG / sqrtG from the grid's reciprocals y = RN(1 / sqrtG); a phiG so small that the
-// quotient might not be normal takes IEEE division
-__device__ __forceinline__ double div_depth(double x, double b, double y) {
-  const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
-  if (e < 257u && x != 0.) return x / b;
-  return ccs_div_const(x, b, y);
 }
 
 namespace {
@@ -169,6 +169,60 @@ __device__ __forceinline__ double central_diff(int op, const double *f, int s, d
   return (-f[-3 * s] + 9. * f[-2 * s] - 45. * f[-s] + 45. * f[s] - 9. * f[2 * s] + f[3 * s]) / (60. * d);
 }
 
+// Sums and products as FMAs: a DADD or DMUL warp instruction holds the FP64 pipe for
+// 19 cycles, a DFMA for 16 (measured, 4-16 warps per SM).  a 1 + b and a b + (-0) are
+// the sum and the product to the last bit and sign; the two constants come from memory,
+// where the compiler cannot see that the FMA could be an addition or a multiplication.
+struct F64Ops {
+  double one, neg0;
+  __device__ __forceinline__ double add(double a, double b) const { return fma(a, one, b); }
+  __device__ __forceinline__ double sub(double a, double b) const { return fma(-b, one, a); }
+  __device__ __forceinline__ double mul(double a, double b) const { return fma(a, b, neg0); }
+  // x / b from y = RN(1 / b), as ccs_div_const
+  __device__ __forceinline__ double div_const(double x, double b, double y) const {
+    const double q0 = mul(x, y);
+    const double r = fma(-q0, b, x);
+    const double q1 = fma(r, y, q0);
+    const unsigned long long t = (unsigned long long)__double_as_longlong(x) << 1;
+    return t - 1ull >= 0xffe0000000000000ull - 1ull ? q0 : q1;
+  }
+};
+
+// phiG / sqrtG from the grid's reciprocals y = RN(1 / sqrtG); a phiG so small that the
+// quotient might not be normal takes IEEE division
+__device__ __forceinline__ double div_depth(const F64Ops &f, double x, double b, double y) {
+  const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
+  if (e < 257u && x != 0.) return x / b;
+  return f.div_const(x, b, y);
+}
+
+// x / b on the integer pipes, b prepared by the host; values whose quotient might leave
+// the normal range (and zeros) take IEEE division
+__device__ __forceinline__ double div_by(double x, const softfp::Divisor &d, double b) {
+  const uint32_t h = (uint32_t)__double2hiint(x);
+  if (((h >> 20) & 0x7ffu) - 400u >= 1200u) return x / b;
+  const double q = softfp::round_double(softfp::div(softfp::unpack(x), d));
+  return __hiloint2double((int)((uint32_t)__double2hiint(q) | (h & 0x80000000u)), __double2loint(q));
+}
+__device__ __forceinline__ double div_by6(double x) {
+  const uint32_t h = (uint32_t)__double2hiint(x);
+  if (((h >> 20) & 0x7ffu) - 400u >= 1200u) return x / 6.;
+  softfp::Quot t = softfp::div3(softfp::unpack(x));
+  t.e -= 1;
+  const double q = softfp::round_double(t);
+  return __hiloint2double((int)((uint32_t)__double2hiint(q) | (h & 0x80000000u)), __double2loint(q));
+}
+
+// -q(-3) + 9 q(-2) - 45 q(-1) + 45 q(1) - 9 q(2) + q(3), left to right
+// (spatial_operators_mod.F90:165,169)
+__device__ __forceinline__ double diff6(const F64Ops &f, const double *q, int s) {
+  double t = f.add(-q[-3 * s], f.mul(9., q[-2 * s]));
+  t = f.sub(t, f.mul(45., q[-s]));
+  t = f.add(t, f.mul(45., q[s]));
+  t = f.sub(t, f.mul(9., q[2 * s]));
+  return f.add(t, q[3 * s]);
+}
+
 // x / 2 of a normal x by its exponent; zeros, infinities, NaNs and values at the
 // bottom of the range take the FP64 multiplication
 __device__ __forceinline__ double half_of(double x) {
@@ -186,6 +240,37 @@ __device__ __forceinline__ bool in_window(double x) {
   return t == 0ull || t - ((unsigned long long)(1023 - 200) << 53) < ((unsigned long long)400 << 53);
 }
 
+// The switches of spatial_operators_mod.F90:348-351 on tau40 = |be0 - be1|, tau41 =
+// |be1 - be2| and mn = min(be): first = (tau40 <= mn && tau41 > mn), last = (tau40 > mn &&
+// tau41 < mn), the differences rounded as FP64 rounds them.  Single precision decides
+// them when both differences are further from mn than its error: the betas as floats
+// relative to the largest exponent, cut to 20 bits (error 2^-20, the largest in [1, 2)), so
+// tau - mn is off by less than 4e-6.  A warp with a closer call takes the FP64 differences.
+__device__ __forceinline__ void switches(const F64Ops &f, double be0, double be1, double be2, long long mn,
+                                         bool &first, bool &last) {
+  const int h0 = __double2hiint(be0), h1 = __double2hiint(be1), h2 = __double2hiint(be2);
+  const int base = (max(max(h0, h1), h2) & 0x7ff00000) - (127 << 20);
+  const float f0 = __int_as_float(max(h0 - base, 0) << 3), f1 = __int_as_float(max(h1 - base, 0) << 3),
+              f2 = __int_as_float(max(h2 - base, 0) << 3);
+  const float fm = fminf(fminf(f0, f1), f2);
+  const float d40 = fabsf(f0 - f1) - fm, d41 = fabsf(f1 - f2) - fm;
+  first = d40 < 0.f && d41 > 0.f;
+  last = d40 > 0.f && d41 < 0.f;
+  if (__any_sync(__activemask(), !(fminf(fabsf(d40), fabsf(d41)) > 1e-5f))) {
+    const long long t40 = abs_bits(f.sub(be0, be1)), t41 = abs_bits(f.sub(be1, be2));
+    first = t40 <= mn && t41 > mn;
+    last = t40 > mn && t41 < mn;
+  }
+}
+
+// a w
+__device__ __forceinline__ double times(double a, softfp::Unp w) {
+  using namespace softfp;
+  const unsigned long long bits = __double_as_longlong(a), sign = bits & 0x8000000000000000ull;
+  const double r = round_double(mul(unpack(a), w));
+  return __longlong_as_double((bits << 1 == 0 ? 0ull : (unsigned long long)__double_as_longlong(r)) | sign);
+}
+
 // One WENO-Z reconstruction (WENO_limiter, spatial_operators_mod.F90:282-361) of a
 // cell's value at one of its two faces, in the reference's order of operations:
 // Q at stride +s for the "+" side (face after the cell), -s for the "-" side, whose
@@ -195,53 +280,55 @@ __device__ __forceinline__ bool in_window(double x) {
 //   ga at the cell: 13/12 (second difference centred there)^2, same orientation
 // (Q/6 and 1/6 Q are exact halves of Q/3 and 1/3 Q; multiplications by 2, 4 and 1/4 are
 // exact and fuse.)  The quotients run on the integer pipes (ccs_softfp.cuh).
-__device__ __forceinline__ double side(const double *Q, int s, const double *G, int SG, int gs, const double *ga,
+__device__ __forceinline__ double side(const F64Ops &f, const double *Q, int s, const double *G, int SG, int gs, const double *ga,
                                        int as) {
   const double q3 = G[5 * SG];
-  const double b0 = fma(-4., Q[-s], Q[-2 * s]) + q3;
-  const double b1 = Q[-s] - Q[s];
-  const double b2 = fma(-4., Q[s], q3) + Q[2 * s];
-  const double be0 = fma(b0 * b0, 0.25, ga[-as]);
-  const double be1 = fma(b1 * b1, 0.25, ga[0]);
-  const double be2 = fma(b2 * b2, 0.25, ga[as]);
-  // the betas are sums of squares (never -0 or negative), the taus absolute values
-  const long long t40 = abs_bits(be0 - be1), t41 = abs_bits(be1 - be2);
-  const double tau5 = fabs(be2 - be0);
+  const double b0 = f.add(fma(-4., Q[-s], Q[-2 * s]), q3);
+  const double b1 = f.sub(Q[-s], Q[s]);
+  const double b2 = f.add(fma(-4., Q[s], q3), Q[2 * s]);
+  const double be0 = fma(f.mul(b0, b0), 0.25, ga[-as]);
+  const double be1 = fma(f.mul(b1, b1), 0.25, ga[0]);
+  const double be2 = fma(f.mul(b2, b2), 0.25, ga[as]);
+  const double tau5 = fabs(f.sub(be2, be0));
   long long mn = __double_as_longlong(be0);
   if (__double_as_longlong(be1) < mn) mn = __double_as_longlong(be1);
   if (__double_as_longlong(be2) < mn) mn = __double_as_longlong(be2);
-  double w0, w1, w2;
-  if (t40 <= mn && t41 > mn) {
-    w0 = 1. / 3.; w1 = 2. / 3.; w2 = 0.;
-  } else if (t40 > mn && t41 < mn) {
-    w0 = 0.; w1 = 2. / 3.; w2 = 1. / 3.;
-  } else {
-    using namespace softfp;
-    const double eps = 1.E-2;
-    const Unp k01{0xccccccccccccd000ull, 1019}, k06{0x9999999999999800ull, 1022}, k03{0x9999999999999800ull, 1021};
+  bool first, last;  // the reference's two switches to fixed weights
+  switches(f, be0, be1, be2, mn, first, last);
+  using namespace softfp;
+  double w0 = first ? 1. / 3. : 0., w1 = 2. / 3., w2 = first ? 0. : 1. / 3.;
+  const double s0 = f.add(f.sub(G[-2 * gs], G[SG - gs]), G[2 * SG]);
+  const double s1 = f.add(fma(-0.5, G[-gs], G[3 * SG]), G[4 * SG + gs]);
+  const double s2 = fma(-0.5, G[4 * SG + 2 * gs], f.add(G[0], G[3 * SG + gs]));
+  if (!first && !last) {
+    // eps + beta: beta itself from 2^48 on (eps is less than half its last place), which
+    // is every beta of the fluxes and phitG
+    double e0 = be0, e1 = be1, e2 = be2;
+    if (__any_sync(__activemask(), mn < 0x42f0000000000000LL)) {
+      const double eps = 1.E-2;
+      e0 = f.add(eps, be0); e1 = f.add(eps, be1); e2 = f.add(eps, be2);
+    }
+    constexpr Unp k01 = constant(0.1), k06 = constant(0.6), k03 = constant(0.3);
     const Unp t = unpack(tau5);  // tau5 = 0 reads as 2^-1023: 1 + tau5 / .. rounds to 1 either way
-    const Unp p0 = one_plus(div(t, divisor(unpack(eps + be0))));
-    const Unp p1 = one_plus(div(t, divisor(unpack(eps + be1))));
-    const Unp p2 = one_plus(div(t, divisor(unpack(eps + be2))));
-    const Unp a0 = mul(p0, k01), a1 = mul(p1, k06), a2 = mul(p2, k03);
-    const Divisor d = divisor(unpack((pack(a0) + pack(a1)) + pack(a2)));
-    w0 = pack(div(a0, d));
-    w1 = pack(div(a1, d));
-    w2 = pack(div(a2, d));
+    const Unp p0 = round_unp(one_plus(div(t, divisor(unpack(e0)))));
+    const Unp p1 = round_unp(one_plus(div(t, divisor(unpack(e1)))));
+    const Unp p2 = round_unp(one_plus(div(t, divisor(unpack(e2)))));
+    const Unp a0 = round_unp(mul(p0, k01)), a1 = round_unp(mul(p1, k06)), a2 = round_unp(mul(p2, k03));
+    const Divisor d = divisor(round_unp(add(round_unp(add(a0, a1)), a2)));
+    w0 = round_double(div(a0, d));
+    w1 = round_double(div(a1, d));
+    w2 = round_double(div(a2, d));
   }
-  const double s0 = (G[-2 * gs] - G[SG - gs]) + G[2 * SG];
-  const double s1 = fma(-0.5, G[-gs], G[3 * SG]) + G[4 * SG + gs];
-  const double s2 = fma(-0.5, G[4 * SG + 2 * gs], G[0] + G[3 * SG + gs]);
-  return fma(s0, w0, 0.) + s1 * w1 + s2 * w2;
+  return f.add(f.add(fma(s0, w0, 0.), f.mul(s1, w1)), f.mul(s2, w2));
 }
 
 // 13/12 a^2 rounded as the reference does: ((a a) 13) / 12
 __device__ __forceinline__ double curvature(double a) {
   using namespace softfp;
   const Unp u = unpack(a);
-  Unp g = div3(mul13(mul(u, u)));
+  Quot g = div3(round_unp(mul13(round_unp(mul(u, u)))));
   g.e -= 2;
-  return a == 0. ? 0. : pack(g);
+  return __double_as_longlong(a) << 1 == 0 ? 0. : round_double(g);
 }
 
 template <class T>
@@ -260,17 +347,18 @@ __device__ __forceinline__ bool is_corner(int i, int j, int N) {
   return (i < 1 || i > N) && (j < 1 || j > N);
 }
 
-__device__ __forceinline__ void store_singles(double *G, int SG, double q) {
+__device__ __forceinline__ void store_singles(const F64Ops &f, double *G, int SG, double q) {
   using namespace softfp;
-  const Unp t = div3(unpack(q));
+  const double t = round_double(div3(unpack(q)));
   const double third = __longlong_as_double(
-      q == 0. ? __double_as_longlong(q)
-              : __double_as_longlong(pack(t)) | (__double_as_longlong(q) & (long long)0x8000000000000000ull));
+      __double_as_longlong(q) << 1 == 0 ? __double_as_longlong(q)
+              : __double_as_longlong(t) | (__double_as_longlong(q) & (long long)0x8000000000000000ull));
   G[0] = third;
-  G[SG] = 7. / 6. * q;
-  G[2 * SG] = 11. / 6. * q;
-  G[3 * SG] = 5. / 6. * q;
-  G[4 * SG] = 1. / 3. * q;
+  constexpr Unp k76 = constant(7. / 6.), k116 = constant(11. / 6.), k56 = constant(5. / 6.), k13 = constant(1. / 3.);
+  G[SG] = times(q, k76);
+  G[2 * SG] = times(q, k116);
+  G[3 * SG] = times(q, k56);
+  G[4 * SG] = times(q, k13);
   G[5 * SG] = fma(2., q, q);
 }
 
@@ -278,8 +366,8 @@ __device__ __forceinline__ void store_singles(double *G, int SG, double q) {
 // rows and QY along the columns (the same array for E and phitG).  rec receives
 // (+) + (-) or, with DIFF, (-) - (+).  nx, ny: the tile's cells inside the panel.
 template <class T, bool SAME, bool DIFF>
-__device__ __forceinline__ void reconstruct(Smem<T> &S, const double *QX, const double *QY, double *rec, int nx,
-                                            int ny, bool slow) {
+__device__ __forceinline__ void reconstruct(Smem<T> &S, const F64Ops &f, const double *QX, const double *QY,
+                                            double *rec, int nx, int ny, bool slow) {
   constexpr int TX = T::TX, TY = T::TY, RX = T::RX, RY = T::RY, RN = T::RN, NLX = T::NLX, NLY = T::NLY;
   constexpr int NFX = T::NFX, NF = T::NF;
   const int tid = threadIdx.x;
@@ -290,60 +378,62 @@ __device__ __forceinline__ void reconstruct(Smem<T> &S, const double *QX, const 
   double *AX = S.scr + (SAME ? NSING * RN : NSING * (NLX + NLY)), *AY = AX + 2 * NLX;
   if (!slow) {
     if constexpr (SAME) {
-      for (int r = tid; r < RN; r += NT) store_singles(GX + r, SGX, QX[r]);
+      for (int r = tid; r < RN; r += NT) store_singles(f, GX + r, SGX, QX[r]);
     } else {
       for (int r = tid; r < NLX + NLY; r += NT) {
         if (r < NLX) {
-          store_singles(GX + r, SGX, QX[3 * RX + r]);
+          store_singles(f, GX + r, SGX, QX[3 * RX + r]);
         } else {
           const int q = r - NLX;
-          store_singles(GY + q, SGY, QY[(q / TX) * RX + q % TX + 3]);
+          store_singles(f, GY + q, SGY, QY[(q / TX) * RX + q % TX + 3]);
         }
       }
     }
     for (int r = tid; r < 2 * (NLX + NLY); r += NT) {
       const bool minus = r >= NLX + NLY;
       const int q = minus ? r - (NLX + NLY) : r;
-      const double *f;
+      const double *z;
       double *o;
       int st;
       bool in;
       if (q < NLX) {
         const int ci = q % RX;
         in = ci >= 1 && ci < RX - 1;
-        f = QX + 3 * RX + q;
+        z = QX + 3 * RX + q;
         st = 1;
         o = AX + (minus ? NLX : 0) + q;
       } else {
         const int k = q - NLX, cj = k / TX;
         in = cj >= 1 && cj < RY - 1;
-        f = QY + cj * RX + k % TX + 3;
+        z = QY + cj * RX + k % TX + 3;
         st = RX;
         o = AY + (minus ? NLY : 0) + k;
       }
       if (in) {
         const int d = minus ? -st : st;
-        *o = curvature(fma(-2., f[0], f[-d]) + f[d]);
+        *o = curvature(f.add(fma(-2., z[0], z[-d]), z[d]));
       }
     }
     __syncthreads();
   }
-  // lanes 2 k and 2 k + 1 take the two sides of one face
+  // lanes 2 k and 2 k + 1 take the two sides of one face; two rounds share one FP64
+  // addition: the even lanes add the first round's faces, the odd lanes the second's
+  double first = 0.;
+  int first_face = -1;
   for (int t0 = tid & ~31; t0 < 2 * NF; t0 += NT) {
     const int t = t0 + (tid & 31), face = t >> 1, minus = t & 1;
     double val = 0.;
     if (t < 2 * NF) {
       bool in;
       int cell, lcell, st, ls;  // the cell in the halo'd tile and on its line's arrays
-      const double *f;
-      const double *G, *A;
+      const double *z, *G, *A;
       if (face < NFX) {
         const int lj = face / (TX + 1), ci = face % (TX + 1) + 2 + minus;
         in = lj < ny && ci - 2 - minus <= nx;
         cell = (lj + 3) * RX + ci;
         lcell = lj * RX + ci;
         st = ls = 1;
-        f = QX;
+        z = QX;
         G = GX + (SAME ? cell : lcell);
         A = AX + (minus ? NLX : 0);
       } else {
@@ -353,22 +443,32 @@ __device__ __forceinline__ void reconstruct(Smem<T> &S, const double *QX, const 
         lcell = cj * TX + li;
         st = RX;
         ls = TX;
-        f = QY;
+        z = QY;
         G = GY + (SAME ? cell : lcell);
         A = AY + (minus ? NLY : 0);
       }
       if (in && ccs_inb(cell - 2 * st, RN, 211) && ccs_inb(cell + 2 * st, RN, 212)) {
-        f += cell;
+        z += cell;
         if (minus) { st = -st; ls = -ls; }
         if (slow)
-          val = minus ? weno5z<-1>(f[2 * st], f[st], f[0], f[-st], f[-2 * st])
-                      : weno5z<1>(f[-2 * st], f[-st], f[0], f[st], f[2 * st]);
+          val = minus ? weno5z<-1>(z[2 * st], z[st], z[0], z[-st], z[-2 * st])
+                      : weno5z<1>(z[-2 * st], z[-st], z[0], z[st], z[2 * st]);
         else
-          val = side(f, st, G, face < NFX ? SGX : SGY, SAME ? st : ls, A + lcell, ls);
+          val = side(f, z, st, G, face < NFX ? SGX : SGY, SAME ? st : ls, A + lcell, ls);
       }
     }
-    const double other = __shfl_xor_sync(0xffffffffu, val, 1);
-    if (!minus && t < 2 * NF && ccs_inb(face, NF, 213)) rec[face] = DIFF ? other - val : val + other;
+    if (t0 + NT < 2 * NF && first_face < 0) {
+      first = val;
+      first_face = face;
+      continue;
+    }
+    const bool two = first_face >= 0;  // uniform in the warp
+    const double o1 = __shfl_xor_sync(0xffffffffu, two ? first : val, 1), o2 = __shfl_xor_sync(0xffffffffu, val, 1);
+    const double plus = minus ? o2 : two ? first : val, neg = minus ? val : o1;
+    const double sum = DIFF ? f.sub(neg, plus) : f.add(plus, neg);
+    const int dst = minus || !two ? face : first_face;
+    if ((two || !minus) && dst < NF && ccs_inb(dst, NF, 213)) rec[dst] = sum;
+    first_face = -1;
   }
   __syncthreads();
 }
@@ -377,7 +477,7 @@ template <class T>
 __global__ void __launch_bounds__(NT, 2)
 f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict__ work, int nwork) {
   constexpr int TX = T::TX, TY = T::TY, RX = T::RX, RN = T::RN, NFX = T::NFX, NF = T::NF;
-  static_assert(T::NT == NT, "phase 3 maps one thread to one cell");
+  static_assert(T::NC <= NT, "phase 3 maps one thread to one cell");
   extern __shared__ __align__(16) double smem_raw[];
   Smem<T> &S = *reinterpret_cast<Smem<T> *>(smem_raw);
   const int tid = threadIdx.x;
@@ -390,6 +490,7 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
     const int i0 = 1 + wi.tx * TX, j0 = 1 + wi.ty * TY;
     const bool ediss = st.ediss != 0;
     const int op = st.op;  // uniform over the work item
+    const F64Ops f{st.one, st.neg0};
 #ifdef CCS_BOUNDS
     // poison the tile arrays: a read of a slot this tile never wrote shows up as NaN
     // in the result (checked build only)
@@ -413,12 +514,12 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
         v = st.in.v[c];
         uC = st.in.uC[c];
         vC = st.in.vC[c];
-        phit = phi + st.m.phis[c];
-        phitG = phit * st.m.sqrtG[c];
-        const double K = half_of(u * uC + v * vC);
-        E = phit + K;
-        Fx = phiG * uC;
-        Fy = phiG * vC;
+        phit = f.add(phi, st.m.phis[c]);
+        phitG = f.mul(phit, st.m.sqrtG[c]);
+        const double K = half_of(f.add(f.mul(u, uC), f.mul(v, vC)));
+        E = f.add(phit, K);
+        Fx = f.mul(phiG, uC);
+        Fy = f.mul(phiG, vC);
         odd = odd || __double_as_longlong(phit) <= 0 || !in_window(phitG) || !in_window(E) || !in_window(Fx) || !in_window(Fy) ||
               !in_window(u) || !in_window(v);
       }
@@ -433,10 +534,10 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
     // ---- phase 2: face reconstructions (weno, :183-277) ---------------------
     // (the central-difference operators have no faces: straight to phase 3)
     if (op == CCS_OP_WENO) {
-    reconstruct<T, false, false>(S, S.Fx, S.Fy, S.rec[0], nx, ny, slow);
-    reconstruct<T, true, false>(S, S.E, S.E, S.rec[1], nx, ny, slow);
-    reconstruct<T, true, true>(S, S.phitG, S.phitG, S.rec[2], nx, ny, slow);
-    if (ediss) reconstruct<T, false, true>(S, S.u, S.v, S.rec[3], nx, ny, slow);
+    reconstruct<T, false, false>(S, f, S.Fx, S.Fy, S.rec[0], nx, ny, slow);
+    reconstruct<T, true, false>(S, f, S.E, S.E, S.rec[1], nx, ny, slow);
+    reconstruct<T, true, true>(S, f, S.phitG, S.phitG, S.rec[2], nx, ny, slow);
+    if (ediss) reconstruct<T, false, true>(S, f, S.u, S.v, S.rec[3], nx, ny, slow);
 
     // ---- phase 2b: Rusanov fluxes at faces (:101-149) ------------------------
     for (int face = tid; face < NF; face += NT) {
@@ -457,11 +558,14 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
         pa = S.phit[r + RX]; pb = S.phit[r];
         lam = st.m.lamy[L.idx(i0 + li, j0 - 1 + fj, p)];
       }
-      const double uBdy = half_of(a + b);
-      const double phitBdy = half_of(pa + pb);
+      const double uBdy = half_of(f.add(a, b));
+      const double phitBdy = half_of(f.add(pa, pb));
       // max(|u - c|, |u + c|) = |u| + c, rounded alike
-      const double cs = sqrt(lam * phitBdy);
-      double mx = fabs(uBdy) + cs;
+      const double c2 = f.mul(lam, phitBdy);
+      const double cs = ((uint32_t)__double2hiint(c2) >> 20) - 400u < 1200u
+                            ? softfp::square_root(softfp::unpack(c2))
+                            : sqrt(c2);
+      double mx = f.add(fabs(uBdy), cs);
       if (slow) {  // (a cell that is not finite keeps the reference's comparison)
         const double e1 = uBdy - cs, e2 = uBdy + cs;
         mx = abs_bits(e2) > abs_bits(e1) ? fabs(e2) : fabs(e1);
@@ -470,8 +574,8 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
       double ES = S.rec[1][face];
       // the never-written u_ext / v_ext slots (CCS_EDISS_ZERO) contribute mx (0 - 0): zero
       // but for a wave speed that is not finite
-      if (ediss || slow) ES = ES - mx * (ediss ? S.rec[3][face] : 0.);
-      S.rec[0][face] = half_of(FS - mx * PD);
+      if (ediss || slow) ES = f.sub(ES, f.mul(mx, ediss ? S.rec[3][face] : 0.));
+      S.rec[0][face] = half_of(f.sub(FS, f.mul(mx, PD)));
       S.rec[1][face] = half_of(ES);
     }
     __syncthreads();
@@ -483,26 +587,20 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
       const int i = i0 + li, j = j0 + lj;
       const int64_t c = L.idx(i, j, p);
       const int rc = (lj + 3) * RX + li + 3;
-      if (i <= N && j <= N && ccs_inb(c, L.field, 221) && ccs_inb(rc + 3 * RX, RN, 222) &&
+      if (tid < T::NC && i <= N && j <= N && ccs_inb(c, L.field, 221) && ccs_inb(rc + 3 * RX, RN, 222) &&
           ccs_inb(NFX + (lj + 1) * TX + li, NF, 223)) {
         double dfluxdx, dEdx, dvdx, dfluxdy, dEdy, dudy;
         if (op == CCS_OP_WENO) {
           const double *FF = S.rec[0], *EF = S.rec[1];
           const int xl = lj * (TX + 1) + li, xr = xl + 1;
           const int yb = NFX + lj * TX + li, yt = yb + TX;
-          // divisions by dx, dy, 60 dx, 60 dy (spatial_operators_mod.F90:153-169) from
-          // their reciprocals, corrected to the IEEE quotients (ccs_div_const)
-          dfluxdx = ccs_div_const(FF[xr] - FF[xl], st.dx, st.rdx);
-          dEdx = ccs_div_const(EF[xr] - EF[xl], st.dx, st.rdx);
-          const double *vr = S.v + (lj + 3) * RX + li;  // v(i-3 .. i+3) at vr[0..6]
-          dvdx = ccs_div_const(-vr[0] + 9. * vr[1] - 45. * vr[2] + 45. * vr[4] - 9. * vr[5] + vr[6], st.dx60,
-                               st.rdx60);
-          dfluxdy = ccs_div_const(FF[yt] - FF[yb], st.dy, st.rdy);
-          dEdy = ccs_div_const(EF[yt] - EF[yb], st.dy, st.rdy);
-          const double *uc = S.u + lj * RX + li + 3;  // u(j-3 .. j+3) at uc[k * RX]
-          dudy = ccs_div_const(-uc[0] + 9. * uc[RX] - 45. * uc[2 * RX] + 45. * uc[4 * RX] - 9. * uc[5 * RX] +
-                                   uc[6 * RX],
-                               st.dy60, st.rdy60);
+          // (spatial_operators_mod.F90:153-169)
+          dfluxdx = div_by(f.sub(FF[xr], FF[xl]), st.by_dx, st.dx);
+          dEdx = div_by(f.sub(EF[xr], EF[xl]), st.by_dx, st.dx);
+          dvdx = div_by(diff6(f, S.v + rc, 1), st.by_dx60, st.dx60);
+          dfluxdy = div_by(f.sub(FF[yt], FF[yb]), st.by_dy, st.dy);
+          dEdy = div_by(f.sub(EF[yt], EF[yb]), st.by_dy, st.dy);
+          dudy = div_by(diff6(f, S.u + rc, RX), st.by_dy60, st.dy60);
         } else {
           dfluxdx = central_diff(op, S.Fx + rc, 1, st.dx);
           dEdx = central_diff(op, S.E + rc, 1, st.dx);
@@ -511,11 +609,11 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
           dEdy = central_diff(op, S.E + rc, RX, st.dy);
           dudy = central_diff(op, S.u + rc, RX, st.dy);
         }
-        const double vort = dvdx - dudy + st.m.sqrtGf[c];
+        const double vort = f.add(f.sub(dvdx, dudy), st.m.sqrtGf[c]);
         const double uCc = S.uC[rc], vCc = S.vC[rc];
-        const double tp = -(dfluxdx + dfluxdy);
-        const double tu = -dEdx + vort * vCc;
-        const double tv = -dEdy - vort * uCc;
+        const double tp = -f.add(dfluxdx, dfluxdy);
+        const double tu = f.add(-dEdx, f.mul(vort, vCc));
+        const double tv = f.sub(-dEdy, f.mul(vort, uCc));
 
         if (st.kind == K_TEND) {
           st.tphiG[c] = tp;
@@ -527,25 +625,25 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
           switch (st.kind) {
             case K_RK4_1:
               st.accphiG[c] = tp; st.accu[c] = tu; st.accv[c] = tv;
-              np = y0p + st.c1 * tp; nu = y0u + st.c1 * tu; nv = y0v + st.c1 * tv;
+              np = f.add(y0p, f.mul(st.c1, tp)); nu = f.add(y0u, f.mul(st.c1, tu)); nv = f.add(y0v, f.mul(st.c1, tv));
               break;
             case K_RK4_2: {
               const double ap = fma(2., tp, st.accphiG[c]);
               const double au = fma(2., tu, st.accu[c]);
               const double av = fma(2., tv, st.accv[c]);
               st.accphiG[c] = ap; st.accu[c] = au; st.accv[c] = av;
-              np = y0p + st.c1 * tp; nu = y0u + st.c1 * tu; nv = y0v + st.c1 * tv;
+              np = f.add(y0p, f.mul(st.c1, tp)); nu = f.add(y0u, f.mul(st.c1, tu)); nv = f.add(y0v, f.mul(st.c1, tv));
               break;
             }
             case K_RK4_4: {
-              const double kp = ccs_div_const(st.accphiG[c] + tp, 6., 1. / 6.);
-              const double ku = ccs_div_const(st.accu[c] + tu, 6., 1. / 6.);
-              const double kv = ccs_div_const(st.accv[c] + tv, 6., 1. / 6.);
-              np = y0p + st.c1 * kp; nu = y0u + st.c1 * ku; nv = y0v + st.c1 * kv;
+              const double kp = div_by6(f.add(st.accphiG[c], tp));
+              const double ku = div_by6(f.add(st.accu[c], tu));
+              const double kv = div_by6(f.add(st.accv[c], tv));
+              np = f.add(y0p, f.mul(st.c1, kp)); nu = f.add(y0u, f.mul(st.c1, ku)); nv = f.add(y0v, f.mul(st.c1, kv));
               break;
             }
             case K_RK3_1:
-              np = y0p + st.c1 * tp; nu = y0u + st.c1 * tu; nv = y0v + st.c1 * tv;
+              np = f.add(y0p, f.mul(st.c1, tp)); nu = f.add(y0u, f.mul(st.c1, tu)); nv = f.add(y0v, f.mul(st.c1, tv));
               break;
             case K_RK3_2: {
               const double ycp = st.in.phiG[c], ycu = S.u[rc], ycv = S.v[rc];
@@ -563,16 +661,16 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
             }
           }
           // correct_bdy_ghost: P2SP (interior), SP2P, cov2contrav, phi = phiG / sqrtG
-          const double zon = st.m.aig11[c] * nu + st.m.aig12[c] * nv;
-          const double mer = st.m.aig21[c] * nu + st.m.aig22[c] * nv;
-          const double u2 = st.m.gia11[c] * zon + st.m.gia12[c] * mer;
-          const double v2 = st.m.gia21[c] * zon + st.m.gia22[c] * mer;
+          const double zon = f.add(f.mul(st.m.aig11[c], nu), f.mul(st.m.aig12[c], nv));
+          const double mer = f.add(f.mul(st.m.aig21[c], nu), f.mul(st.m.aig22[c], nv));
+          const double u2 = f.add(f.mul(st.m.gia11[c], zon), f.mul(st.m.gia12[c], mer));
+          const double v2 = f.add(f.mul(st.m.gia21[c], zon), f.mul(st.m.gia22[c], mer));
           st.out.phiG[c] = np;
           st.out.u[c] = u2;
           st.out.v[c] = v2;
-          st.out.uC[c] = st.m.ig11[c] * u2 + st.m.ig12[c] * v2;
-          st.out.vC[c] = st.m.ig21[c] * u2 + st.m.ig22[c] * v2;
-          st.out.phi[c] = div_depth(np, st.m.sqrtG[c], st.m.rsqrtG[c]);
+          st.out.uC[c] = f.add(f.mul(st.m.ig11[c], u2), f.mul(st.m.ig12[c], v2));
+          st.out.vC[c] = f.add(f.mul(st.m.ig21[c], u2), f.mul(st.m.ig22[c], v2));
+          st.out.phi[c] = div_depth(f, np, st.m.sqrtG[c], st.m.rsqrtG[c]);
           if (st.zonal) {
             st.zonal[c] = zon;
             st.merid[c] = mer;
@@ -591,14 +689,14 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
             if (!ccs_inb(e, (long long)24 * h * N, 224)) continue;
             const int64_t d = st.m.push[e];
             if (!ccs_inb(d, L.field, 225)) continue;
-            const double ud = st.m.gia11[d] * zon + st.m.gia12[d] * mer;
-            const double vd = st.m.gia21[d] * zon + st.m.gia22[d] * mer;
+            const double ud = f.add(f.mul(st.m.gia11[d], zon), f.mul(st.m.gia12[d], mer));
+            const double vd = f.add(f.mul(st.m.gia21[d], zon), f.mul(st.m.gia22[d], mer));
             st.out.phiG[d] = np;
             st.out.u[d] = ud;
             st.out.v[d] = vd;
-            st.out.uC[d] = st.m.ig11[d] * ud + st.m.ig12[d] * vd;
-            st.out.vC[d] = st.m.ig21[d] * ud + st.m.ig22[d] * vd;
-            st.out.phi[d] = div_depth(np, st.m.sqrtG[d], st.m.rsqrtG[d]);
+            st.out.uC[d] = f.add(f.mul(st.m.ig11[d], ud), f.mul(st.m.ig12[d], vd));
+            st.out.vC[d] = f.add(f.mul(st.m.ig21[d], ud), f.mul(st.m.ig22[d], vd));
+            st.out.phi[d] = div_depth(f, np, st.m.sqrtG[d], st.m.rsqrtG[d]);
             if (st.zonal) {
               st.zonal[d] = zon;
               st.merid[d] = mer;

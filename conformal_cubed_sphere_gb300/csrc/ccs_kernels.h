@@ -7,6 +7,7 @@
 #include <cstdint>
 
 #include "ccs_internal.h"
+#include "ccs_softfp.cuh"
 
 namespace ccs {
 
@@ -54,9 +55,10 @@ struct F64Stage {
   double *zonal, *merid;  // sphere winds of Y_{k+1} when non-null
   double *tphiG, *tu, *tv;
   double dx, dy, dx60, dy60, c1;
-  double rdx, rdy, rdx60, rdy60;  // RN(1 / dx) etc.: the divisions by them are corrected to IEEE
+  softfp::Divisor by_dx, by_dy, by_dx60, by_dy60;
   int kind, ediss;
   int op;  // CCS_OP_WENO, or the central-difference order 2 / 4 / 6
+  double one = 1., neg0 = -0.;  // the constants of F64Ops, read at run time on purpose
 };
 
 // Mixed lane: one instance's stage launch.
