@@ -250,10 +250,11 @@ static int build_mesh(ccs_handle *h, const ccs_mesh_view *mv) {
   const Layout &L = h->L;
   const size_t nref = (size_t)L.nh * L.nh * 6;
   const size_t nf = (size_t)L.field;
-  // FP64 arrays: sqrtG phis f ig11 ig12 ig21 ig22 aig11..22 gia11..22 sqrtGf rsqrtG lamx lamy
-  constexpr int na = 19;
-  CCS_TRY(h, cudaMalloc(&dm->buf64, na * nf * sizeof(double)));
-  CCS_TRY(h, cudaMemsetAsync(dm->buf64, 0, na * nf * sizeof(double), h->stream));
+  // FP64 arrays: sqrtG phis f ig11 ig12 ig21 ig22 aig11..22 gia11..22 from the host, and
+  // sqrtGf rsqrtG lamx lamy formed from them on the device
+  constexpr int na = 15, nd = 4;
+  CCS_TRY(h, cudaMalloc(&dm->buf64, (na + nd) * nf * sizeof(double)));
+  CCS_TRY(h, cudaMemsetAsync(dm->buf64, 0, (na + nd) * nf * sizeof(double), h->stream));
   std::vector<double> tmp(na * nref, 0.);
   double *t[na];
   for (int k = 0; k < na; k++) t[k] = tmp.data() + k * nref;
@@ -271,17 +272,7 @@ static int build_mesh(ccs_handle *h, const ccs_mesh_view *mv) {
     t[7][c] = M[0]; t[8][c] = M[2]; t[9][c] = M[1]; t[10][c] = M[3];
     matmul22(&mv->matrixG[4 * c], &mv->matrixIA[4 * c], M);  // projection_mod.F90:71
     t[11][c] = M[0]; t[12][c] = M[2]; t[13][c] = M[1]; t[14][c] = M[3];
-    t[15][c] = mv->sqrtG[c] * mv->f[c];
-    t[16][c] = 1. / mv->sqrtG[c];
   }
-  const size_t nh = L.nh;
-  for (int p = 0; p < 6; p++)  // face means (spatial_operators_mod.F90:113-114, 138-139)
-    for (size_t j = 0; j < nh; j++)
-      for (size_t i = 0; i < nh; i++) {
-        const size_t c = i + nh * (j + nh * p);
-        if (i + 1 < nh) t[17][c] = 0.5 * (mv->matrixIG[4 * (c + 1)] + mv->matrixIG[4 * c]);
-        if (j + 1 < nh) t[18][c] = 0.5 * (mv->matrixIG[4 * (c + nh) + 3] + mv->matrixIG[4 * c + 3]);
-      }
   for (int k = 0; k < na; k++) {
     int rc = upload_field(h, dm->buf64 + k * nf, t[k]);
     if (rc) return rc;
@@ -292,6 +283,7 @@ static int build_mesh(ccs_handle *h, const ccs_mesh_view *mv) {
   dm->m64.aig11 = b + 7 * nf; dm->m64.aig12 = b + 8 * nf; dm->m64.aig21 = b + 9 * nf; dm->m64.aig22 = b + 10 * nf;
   dm->m64.gia11 = b + 11 * nf; dm->m64.gia12 = b + 12 * nf; dm->m64.gia21 = b + 13 * nf; dm->m64.gia22 = b + 14 * nf;
   dm->m64.sqrtGf = b + 15 * nf; dm->m64.rsqrtG = b + 16 * nf; dm->m64.lamx = b + 17 * nf; dm->m64.lamy = b + 18 * nf;
+  CCS_TRY(h, launch_f64_mesh_products(L, dm->m64, b + 15 * nf, h->stream));
   std::vector<int32_t> push;
   if (!build_push_table(L, push)) {
     h->err = "ghost tables are inconsistent";

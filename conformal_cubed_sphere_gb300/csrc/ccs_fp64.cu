@@ -38,10 +38,13 @@ namespace {
 // arrays of single-cell products of a reconstructed field (see side)
 constexpr int NSING = 6;
 
-// a tile of TX x TY cells; phase 3 maps one thread to one cell
-template <int TX_, int TY_>
+// A tile of TX x TY cells worked on by NT threads, CTAS of them resident on an SM; phase
+// 3 maps one thread to one cell.  The tile is one of the PX / TX x PY / TY parts of a work
+// item of PX x PY cells (the item itself unless a launch is split).
+template <int TX_, int TY_, int NT_, int CTAS_, int PX_ = TX_, int PY_ = TY_>
 struct F64Tile {
-  static constexpr int TX = TX_, TY = TY_, NC = TX * TY;
+  static constexpr int TX = TX_, TY = TY_, NC = TX * TY, NT = NT_, CTAS = CTAS_;
+  static constexpr int SX = PX_ / TX, SY = PY_ / TY, PX = PX_, PY = PY_;
   static constexpr int RX = TX + 6, RY = TY + 6, RN = RX * RY;
   static constexpr int NFX = TY * (TX + 1), NFY = (TY + 1) * TX, NF = NFX + NFY;
   // cells of the lines through the tile: rows of RX cells, columns of RY
@@ -49,11 +52,6 @@ struct F64Tile {
   static constexpr int NSCR_F = (NSING + 2) * (NLX + NLY), NSCR_E = NSING * RN + 2 * (NLX + NLY);
   static constexpr int NSCR = NSCR_F > NSCR_E ? NSCR_F : NSCR_E;
 };
-// 12 warps and two CTAs an SM (80 registers): the FP64 pipe is shared by the whole SM,
-// and a warp holds it for a fraction of its time (C384 stage: 8 warps 1023 us, 12 warps
-// 989, 16 warps, which spill, 1032)
-constexpr int NT = 384;
-
 }  // namespace
 
 // x / b for a divisor fixed in advance — the constants 3, 6, 12 of the reference
@@ -341,6 +339,7 @@ struct Smem {
   // per-cell products of the fields of one pass: either fields of their own on the rows
   // and columns, or one field on the halo'd tile with curvatures on rows and columns
   double scr[T::NSCR];
+  F64Stage st;  // the work item's stage descriptor
 };
 
 __device__ __forceinline__ bool is_corner(int i, int j, int N) {
@@ -369,7 +368,7 @@ template <class T, bool SAME, bool DIFF>
 __device__ __forceinline__ void reconstruct(Smem<T> &S, const F64Ops &f, const double *QX, const double *QY,
                                             double *rec, int nx, int ny, bool slow) {
   constexpr int TX = T::TX, TY = T::TY, RX = T::RX, RY = T::RY, RN = T::RN, NLX = T::NLX, NLY = T::NLY;
-  constexpr int NFX = T::NFX, NF = T::NF;
+  constexpr int NFX = T::NFX, NF = T::NF, NT = T::NT;
   const int tid = threadIdx.x;
   // products: [NSING] arrays on the halo'd tile (SAME) or on the rows / columns, then
   // the curvatures of the "+" and "-" orientation on the rows and on the columns
@@ -473,28 +472,62 @@ __device__ __forceinline__ void reconstruct(Smem<T> &S, const F64Ops &f, const d
   __syncthreads();
 }
 
+// Writes cell c of the stage's output from its phiG and sphere wind: the covariant and
+// contravariant wind by the cell's own metric, and phi.
+__device__ __forceinline__ void complete(const F64Ops &f, const F64Stage &st, int64_t c, double phiG, double zon,
+                                         double mer) {
+  const MeshF64 &m = st.m;
+  const double g11 = __ldg(m.gia11 + c), g12 = __ldg(m.gia12 + c), g21 = __ldg(m.gia21 + c), g22 = __ldg(m.gia22 + c);
+  const double i11 = __ldg(m.ig11 + c), i12 = __ldg(m.ig12 + c), i21 = __ldg(m.ig21 + c), i22 = __ldg(m.ig22 + c);
+  const double sg = __ldg(m.sqrtG + c), rsg = __ldg(m.rsqrtG + c);
+  const double u = f.add(f.mul(g11, zon), f.mul(g12, mer));
+  const double v = f.add(f.mul(g21, zon), f.mul(g22, mer));
+  const double uC = f.add(f.mul(i11, u), f.mul(i12, v));
+  const double vC = f.add(f.mul(i21, u), f.mul(i22, v));
+  const double phi = div_depth(f, phiG, sg, rsg);
+  st.out.phiG[c] = phiG;
+  st.out.u[c] = u;
+  st.out.v[c] = v;
+  st.out.uC[c] = uC;
+  st.out.vC[c] = vC;
+  st.out.phi[c] = phi;
+  if (st.zonal) {
+    st.zonal[c] = zon;
+    st.merid[c] = mer;
+  }
+}
+
 template <class T>
-__global__ void __launch_bounds__(NT, 2)
+__global__ void __launch_bounds__(T::NT, T::CTAS)
 f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict__ work, int nwork) {
-  constexpr int TX = T::TX, TY = T::TY, RX = T::RX, RN = T::RN, NFX = T::NFX, NF = T::NF;
+  constexpr int TX = T::TX, TY = T::TY, RX = T::RX, RN = T::RN, NFX = T::NFX, NF = T::NF, NT = T::NT;
+  constexpr int PARTS = T::SX * T::SY;
   static_assert(T::NC <= NT, "phase 3 maps one thread to one cell");
   extern __shared__ __align__(16) double smem_raw[];
   Smem<T> &S = *reinterpret_cast<Smem<T> *>(smem_raw);
   const int tid = threadIdx.x;
 
   for (int w = blockIdx.x; w < nwork; w += gridDim.x) {
-    const WorkItem wi = work[w];
-    const F64Stage &st = stages[wi.inst];
+    const WorkItem wi = work[w / PARTS];
+    const F64Stage &st = S.st;
+    {  // (the loop's last barrier is behind every thread's use of the previous one)
+      const uint64_t *src = reinterpret_cast<const uint64_t *>(stages + wi.inst);
+      uint64_t *dst = reinterpret_cast<uint64_t *>(&S.st);
+      static_assert(sizeof(F64Stage) % sizeof(uint64_t) == 0, "copied in words");
+      for (int k = tid; k < (int)(sizeof(F64Stage) / sizeof(uint64_t)); k += NT) dst[k] = __ldg(src + k);
+    }
+    __syncthreads();
     const Layout L = st.L;
     const int N = L.N, p = wi.panel;
-    const int i0 = 1 + wi.tx * TX, j0 = 1 + wi.ty * TY;
+    const int i0 = 1 + wi.tx * T::PX + w % T::SX * TX, j0 = 1 + wi.ty * T::PY + w / T::SX % T::SY * TY;
+    if (i0 > N || j0 > N) continue;  // (a part beyond the panel's edge)
     const bool ediss = st.ediss != 0;
     const int op = st.op;  // uniform over the work item
     const F64Ops f{st.one, st.neg0};
 #ifdef CCS_BOUNDS
     // poison the tile arrays: a read of a slot this tile never wrote shows up as NaN
     // in the result (checked build only)
-    for (int k = tid; k < (int)(sizeof(S) / sizeof(double)); k += NT)
+    for (int k = tid; k < (int)((sizeof(S) - sizeof(S.st)) / sizeof(double)); k += NT)
       smem_raw[k] = __longlong_as_double(0x7ff8000000000000LL);
     __syncthreads();
 #endif
@@ -509,13 +542,13 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
       double phit = 0., phitG = 0., E = 0., Fx = 0., Fy = 0., uC = 0., vC = 0., u = 0., v = 0.;
       const int64_t c = L.idx(i, j, p);
       if (i >= -2 && i <= N + 3 && j >= -2 && j <= N + 3 && !is_corner(i, j, N) && ccs_inb(c, L.field, 201)) {
-        const double phiG = st.in.phiG[c], phi = st.in.phi[c];
-        u = st.in.u[c];
-        v = st.in.v[c];
-        uC = st.in.uC[c];
-        vC = st.in.vC[c];
-        phit = f.add(phi, st.m.phis[c]);
-        phitG = f.mul(phit, st.m.sqrtG[c]);
+        const double phiG = __ldg(st.in.phiG + c), phi = __ldg(st.in.phi + c);
+        u = __ldg(st.in.u + c);
+        v = __ldg(st.in.v + c);
+        uC = __ldg(st.in.uC + c);
+        vC = __ldg(st.in.vC + c);
+        phit = f.add(phi, __ldg(st.m.phis + c));
+        phitG = f.mul(phit, __ldg(st.m.sqrtG + c));
         const double K = half_of(f.add(f.mul(u, uC), f.mul(v, vC)));
         E = f.add(phit, K);
         Fx = f.mul(phiG, uC);
@@ -548,7 +581,7 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
         if (i0 - 1 + fi > N || j0 + lj > N || !ccs_inb(r + 1, RN, 214)) continue;
         a = S.uC[r + 1]; b = S.uC[r];
         pa = S.phit[r + 1]; pb = S.phit[r];
-        lam = st.m.lamx[L.idx(i0 - 1 + fi, j0 + lj, p)];
+        lam = __ldg(st.m.lamx + L.idx(i0 - 1 + fi, j0 + lj, p));
       } else {
         const int fy = face - NFX;
         const int li = fy % TX, fj = fy / TX;
@@ -556,7 +589,7 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
         if (i0 + li > N || j0 - 1 + fj > N || !ccs_inb(r + RX, RN, 215)) continue;
         a = S.vC[r + RX]; b = S.vC[r];
         pa = S.phit[r + RX]; pb = S.phit[r];
-        lam = st.m.lamy[L.idx(i0 + li, j0 - 1 + fj, p)];
+        lam = __ldg(st.m.lamy + L.idx(i0 + li, j0 - 1 + fj, p));
       }
       const double uBdy = half_of(f.add(a, b));
       const double phitBdy = half_of(f.add(pa, pb));
@@ -582,6 +615,7 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
     }  // op == CCS_OP_WENO
 
     // ---- phase 3: tendencies, stage update, boundary correction --------------
+    double *new_phiG = S.scr, *new_zon = S.scr + T::NC, *new_mer = S.scr + 2 * T::NC;  // for the push
     {
       const int li = tid % TX, lj = tid / TX;
       const int i = i0 + li, j = j0 + lj;
@@ -589,6 +623,17 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
       const int rc = (lj + 3) * RX + li + 3;
       if (tid < T::NC && i <= N && j <= N && ccs_inb(c, L.field, 221) && ccs_inb(rc + 3 * RX, RN, 222) &&
           ccs_inb(NFX + (lj + 1) * TX + li, NF, 223)) {
+        // every global operand before the first store, so that the loads overlap
+        const int kind = st.kind;
+        const double sgf = __ldg(st.m.sqrtGf + c);
+        double y0[3] = {0., 0., 0.}, ac[3] = {0., 0., 0.};
+        if (kind != K_TEND) {
+          y0[0] = st.y0phiG[c]; y0[1] = st.y0u[c]; y0[2] = st.y0v[c];
+          if (kind == K_RK4_2 || kind == K_RK4_4) { ac[0] = st.accphiG[c]; ac[1] = st.accu[c]; ac[2] = st.accv[c]; }
+          if (kind == K_RK3_2 || kind == K_RK3_3) { ac[0] = __ldg(st.in.phiG + c); ac[1] = S.u[rc]; ac[2] = S.v[rc]; }
+        }
+        const double a11 = __ldg(st.m.aig11 + c), a12 = __ldg(st.m.aig12 + c), a21 = __ldg(st.m.aig21 + c),
+                     a22 = __ldg(st.m.aig22 + c);
         double dfluxdx, dEdx, dvdx, dfluxdy, dEdy, dudy;
         if (op == CCS_OP_WENO) {
           const double *FF = S.rec[0], *EF = S.rec[1];
@@ -609,100 +654,69 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
           dEdy = central_diff(op, S.E + rc, RX, st.dy);
           dudy = central_diff(op, S.u + rc, RX, st.dy);
         }
-        const double vort = f.add(f.sub(dvdx, dudy), st.m.sqrtGf[c]);
+        const double vort = f.add(f.sub(dvdx, dudy), sgf);
         const double uCc = S.uC[rc], vCc = S.vC[rc];
-        const double tp = -f.add(dfluxdx, dfluxdy);
-        const double tu = f.add(-dEdx, f.mul(vort, vCc));
-        const double tv = f.sub(-dEdy, f.mul(vort, uCc));
+        const double t[3] = {-f.add(dfluxdx, dfluxdy), f.add(-dEdx, f.mul(vort, vCc)), f.sub(-dEdy, f.mul(vort, uCc))};
 
-        if (st.kind == K_TEND) {
-          st.tphiG[c] = tp;
-          st.tu[c] = tu;
-          st.tv[c] = tv;
+        if (kind == K_TEND) {
+          st.tphiG[c] = t[0];
+          st.tu[c] = t[1];
+          st.tv[c] = t[2];
         } else {
-          const double y0p = st.y0phiG[c], y0u = st.y0u[c], y0v = st.y0v[c];
-          double np, nu, nv;
-          switch (st.kind) {
-            case K_RK4_1:
-              st.accphiG[c] = tp; st.accu[c] = tu; st.accv[c] = tv;
-              np = f.add(y0p, f.mul(st.c1, tp)); nu = f.add(y0u, f.mul(st.c1, tu)); nv = f.add(y0v, f.mul(st.c1, tv));
-              break;
-            case K_RK4_2: {
-              const double ap = fma(2., tp, st.accphiG[c]);
-              const double au = fma(2., tu, st.accu[c]);
-              const double av = fma(2., tv, st.accv[c]);
-              st.accphiG[c] = ap; st.accu[c] = au; st.accv[c] = av;
-              np = f.add(y0p, f.mul(st.c1, tp)); nu = f.add(y0u, f.mul(st.c1, tu)); nv = f.add(y0v, f.mul(st.c1, tv));
-              break;
-            }
-            case K_RK4_4: {
-              const double kp = div_by6(f.add(st.accphiG[c], tp));
-              const double ku = div_by6(f.add(st.accu[c], tu));
-              const double kv = div_by6(f.add(st.accv[c], tv));
-              np = f.add(y0p, f.mul(st.c1, kp)); nu = f.add(y0u, f.mul(st.c1, ku)); nv = f.add(y0v, f.mul(st.c1, kv));
-              break;
-            }
-            case K_RK3_1:
-              np = f.add(y0p, f.mul(st.c1, tp)); nu = f.add(y0u, f.mul(st.c1, tu)); nv = f.add(y0v, f.mul(st.c1, tv));
-              break;
-            case K_RK3_2: {
-              const double ycp = st.in.phiG[c], ycu = S.u[rc], ycv = S.v[rc];
-              np = 0.75 * y0p + 0.25 * ycp + st.c1 * tp;
-              nu = 0.75 * y0u + 0.25 * ycu + st.c1 * tu;
-              nv = 0.75 * y0v + 0.25 * ycv + st.c1 * tv;
-              break;
-            }
-            default: {  // K_RK3_3
-              const double ycp = st.in.phiG[c], ycu = S.u[rc], ycv = S.v[rc];
-              np = y0p / 3. + 2. / 3. * ycp + st.c1 * tp;
-              nu = y0u / 3. + 2. / 3. * ycu + st.c1 * tu;
-              nv = y0v / 3. + 2. / 3. * ycv + st.c1 * tv;
-              break;
-            }
+          double n[3];
+          if (kind == K_RK4_2)
+#pragma unroll
+            for (int q = 0; q < 3; q++) ac[q] = fma(2., t[q], ac[q]);
+#pragma unroll
+          for (int q = 0; q < 3; q++) {
+            if (kind == K_RK4_4)
+              n[q] = f.add(y0[q], f.mul(st.c1, div_by6(f.add(ac[q], t[q]))));
+            else if (kind == K_RK3_2)
+              n[q] = f.add(f.add(f.mul(0.75, y0[q]), f.mul(0.25, ac[q])), f.mul(st.c1, t[q]));
+            else if (kind == K_RK3_3)
+              n[q] = f.add(f.add(f.div_const(y0[q], 3., 1. / 3.), f.mul(2. / 3., ac[q])), f.mul(st.c1, t[q]));
+            else
+              n[q] = f.add(y0[q], f.mul(st.c1, t[q]));
           }
           // correct_bdy_ghost: P2SP (interior), SP2P, cov2contrav, phi = phiG / sqrtG
-          const double zon = f.add(f.mul(st.m.aig11[c], nu), f.mul(st.m.aig12[c], nv));
-          const double mer = f.add(f.mul(st.m.aig21[c], nu), f.mul(st.m.aig22[c], nv));
-          const double u2 = f.add(f.mul(st.m.gia11[c], zon), f.mul(st.m.gia12[c], mer));
-          const double v2 = f.add(f.mul(st.m.gia21[c], zon), f.mul(st.m.gia22[c], mer));
-          st.out.phiG[c] = np;
-          st.out.u[c] = u2;
-          st.out.v[c] = v2;
-          st.out.uC[c] = f.add(f.mul(st.m.ig11[c], u2), f.mul(st.m.ig12[c], v2));
-          st.out.vC[c] = f.add(f.mul(st.m.ig21[c], u2), f.mul(st.m.ig22[c], v2));
-          st.out.phi[c] = div_depth(f, np, st.m.sqrtG[c], st.m.rsqrtG[c]);
-          if (st.zonal) {
-            st.zonal[c] = zon;
-            st.merid[c] = mer;
+          const double zon = f.add(f.mul(a11, n[1]), f.mul(a12, n[2]));
+          const double mer = f.add(f.mul(a21, n[1]), f.mul(a22, n[2]));
+          new_phiG[tid] = n[0]; new_zon[tid] = zon; new_mer[tid] = mer;
+          if (kind == K_RK4_1) {
+            st.accphiG[c] = t[0]; st.accu[c] = t[1]; st.accv[c] = t[2];
+          } else if (kind == K_RK4_2) {
+            st.accphiG[c] = ac[0]; st.accu[c] = ac[1]; st.accv[c] = ac[2];
           }
-          // ghost push: this cell's value lands in the halo strip of each edge it is
-          // within `halo` of (two strips near a panel corner)
-          const int h = L.h;
-          for (int side = 0; side < 4; side++) {
-            int k, m;
-            if (side == 0) { k = i; m = j; }
-            else if (side == 1) { k = N + 1 - i; m = j; }
-            else if (side == 2) { k = j; m = i; }
-            else { k = N + 1 - j; m = i; }
-            if (k > h) continue;
-            const int64_t e = ((int64_t)p * 4 + side) * h * N + (int64_t)(k - 1) * N + (m - 1);
-            if (!ccs_inb(e, (long long)24 * h * N, 224)) continue;
-            const int64_t d = st.m.push[e];
-            if (!ccs_inb(d, L.field, 225)) continue;
-            const double ud = f.add(f.mul(st.m.gia11[d], zon), f.mul(st.m.gia12[d], mer));
-            const double vd = f.add(f.mul(st.m.gia21[d], zon), f.mul(st.m.gia22[d], mer));
-            st.out.phiG[d] = np;
-            st.out.u[d] = ud;
-            st.out.v[d] = vd;
-            st.out.uC[d] = f.add(f.mul(st.m.ig11[d], ud), f.mul(st.m.ig12[d], vd));
-            st.out.vC[d] = f.add(f.mul(st.m.ig21[d], ud), f.mul(st.m.ig22[d], vd));
-            st.out.phi[d] = div_depth(f, np, st.m.sqrtG[d], st.m.rsqrtG[d]);
-            if (st.zonal) {
-              st.zonal[d] = zon;
-              st.merid[d] = mer;
-            }
-          }
+          complete(f, st, c, n[0], zon, mer);
         }
+      }
+    }
+    __syncthreads();
+
+    // ---- phase 4: ghost push of the part's edge strips ------------------------
+    // A cell within `halo` of a panel edge lands in that edge's halo strip (two strips
+    // near a panel corner).  The strip cells of the part, strip by strip (0 left, 1
+    // right, 2 below, 3 above), are dealt out to all threads.
+    if (st.kind != K_TEND) {
+      const int h = L.h, ie = i0 + nx - 1, je = j0 + ny - 1;
+      const int xlo1 = max(i0, N - h + 1), xlo3 = max(j0, N - h + 1);
+      const int o1 = max(min(ie, h) - i0 + 1, 0) * ny;
+      const int o2 = o1 + max(ie - xlo1 + 1, 0) * ny;
+      const int o3 = o2 + max(min(je, h) - j0 + 1, 0) * nx;
+      const int o4 = o3 + max(je - xlo3 + 1, 0) * nx;
+      for (int t = tid; t < o4; t += NT) {
+        const int sd = (t >= o1) + (t >= o2) + (t >= o3);
+        const int q = t - (sd == 0 ? 0 : sd == 1 ? o1 : sd == 2 ? o2 : o3);
+        const int na = sd < 2 ? ny : nx;
+        const int x = (sd == 0 ? i0 : sd == 1 ? xlo1 : sd == 2 ? j0 : xlo3) + q / na, m = (sd < 2 ? j0 : i0) + q % na;
+        const int k = (sd == 0 || sd == 2) ? x : N + 1 - x;
+        const int i = sd < 2 ? x : m, j = sd < 2 ? m : x;
+        const int64_t e = ((int64_t)p * 4 + sd) * h * N + (int64_t)(k - 1) * N + (m - 1);
+        if (!ccs_inb(e, (long long)24 * h * N, 224)) continue;
+        const int64_t d = __ldg(st.m.push + e);
+        const int cell = (j - j0) * TX + i - i0;
+        if (!ccs_inb(d, L.field, 225) || !ccs_inb(cell, T::NC, 226)) continue;
+        complete(f, st, d, new_phiG[cell], new_zon[cell], new_mer[cell]);
       }
     }
     __syncthreads();
@@ -743,9 +757,15 @@ cudaError_t launch_div_const_check(const double *x, int64_t n, double b, double 
 
 namespace {
 
-using F64T0 = F64Tile<32, 8>;
-using F64T1 = F64Tile<16, 16>;
-using F64T2 = F64Tile<64, 4>;
+// 12 warps and two CTAs an SM (80 registers): the FP64 pipe is shared by the whole SM,
+// and a warp holds it for a fraction of its time (C384 stage: 8 warps 1023 us, 12 warps
+// 989, 16 warps, which spill, 1032)
+using F64T0 = F64Tile<32, 8, 384, 2>;
+using F64T1 = F64Tile<16, 16, 384, 2>;
+using F64T2 = F64Tile<64, 4, 384, 1>;
+// parts of 8 x 8 cells: nine warps hold all its face sides at once
+using F64S0 = F64Tile<8, 8, 288, 2, 32, 8>;
+using F64S1 = F64Tile<8, 8, 288, 2, 16, 16>;
 
 template <class T>
 constexpr int f64_smem_bytes() {
@@ -758,7 +778,7 @@ int f64_grid_for(int device) {
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
   constexpr int smem = f64_smem_bytes<T>();
   cudaFuncSetAttribute(f64_stage_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f64_stage_kernel<T>, NT, smem);
+  cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f64_stage_kernel<T>, T::NT, smem);
   if (per < 1) per = 1;
   return sms * per;
 }
@@ -771,8 +791,15 @@ cudaError_t f64_launch(const F64Stage *d_stages, const WorkItem *d_work, int nwo
   if (e != cudaSuccess) return e;
   if (grid > nwork) grid = nwork;
   if (grid < 1) return cudaSuccess;
-  f64_stage_kernel<T><<<grid, NT, smem, s>>>(d_stages, d_work, nwork);
+  f64_stage_kernel<T><<<grid, T::NT, smem, s>>>(d_stages, d_work, nwork);
   return cudaGetLastError();
+}
+
+// the same work items in parts, one CTA each
+template <class T>
+cudaError_t f64_launch_parts(const F64Stage *d_stages, const WorkItem *d_work, int nwork, cudaStream_t s) {
+  const int parts = nwork * T::SX * T::SY;
+  return f64_launch<T>(d_stages, d_work, parts, parts, s);
 }
 
 static_assert(F64T0::TX == kF64Tiles[0].tx && F64T0::TY == kF64Tiles[0].ty, "tile table");
@@ -789,13 +816,42 @@ int f64_max_grid(int var, int device) {
   }
 }
 
+// A launch whose items in four parts still fit the resident CTAs (grid) runs in parts: the
+// 256 cells of an item take one CTA 54 us whatever the number of items, its parts of 64
+// cells 24 us on an SM of their own and 30 us two to an SM (C24: 61 -> 24 us a stage, C48
+// 61 -> 30; C64, with 96 items, 54 us whole and 58 in parts).  64 x 4 items have no such parts.
 cudaError_t launch_f64_stage(int var, const F64Stage *d_stages, const WorkItem *d_work, int nwork, int grid,
                              cudaStream_t s) {
+  const bool split = var != 2 && 4 * nwork <= grid;
   switch (var) {
-    case 1: return f64_launch<F64T1>(d_stages, d_work, nwork, grid, s);
+    case 1:
+      return split ? f64_launch_parts<F64S1>(d_stages, d_work, nwork, s)
+                   : f64_launch<F64T1>(d_stages, d_work, nwork, grid, s);
     case 2: return f64_launch<F64T2>(d_stages, d_work, nwork, grid, s);
-    default: return f64_launch<F64T0>(d_stages, d_work, nwork, grid, s);
+    default:
+      return split ? f64_launch_parts<F64S0>(d_stages, d_work, nwork, s)
+                   : f64_launch<F64T0>(d_stages, d_work, nwork, grid, s);
   }
+}
+
+// Products of static metric terms, each in the order the operator forms it: sqrtG f,
+// 1 / sqrtG, and the face means of the wave-speed metric
+// (spatial_operators_mod.F90:113-114, 138-139, 171).
+__global__ void mesh_products_kernel(Layout L, MeshF64 m, double *__restrict__ out) {
+  const int64_t n = (int64_t)L.nh * L.nh * 6;
+  for (int64_t q = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; q < n; q += (int64_t)gridDim.x * blockDim.x) {
+    const int ia = (int)(q % L.nh), ja = (int)((q / L.nh) % L.nh), p = (int)(q / ((int64_t)L.nh * L.nh));
+    const int64_t c = ia + (int64_t)L.pitch * ja + L.panel * p;
+    out[c] = m.sqrtG[c] * m.f[c];
+    out[L.field + c] = 1. / m.sqrtG[c];
+    if (ia + 1 < L.nh) out[2 * L.field + c] = 0.5 * (m.ig11[c + 1] + m.ig11[c]);
+    if (ja + 1 < L.nh) out[3 * L.field + c] = 0.5 * (m.ig22[c + L.pitch] + m.ig22[c]);
+  }
+}
+
+cudaError_t launch_f64_mesh_products(const Layout &L, const MeshF64 &m, double *out, cudaStream_t s) {
+  mesh_products_kernel<<<1024, 256, 0, s>>>(L, m, out);
+  return cudaGetLastError();
 }
 
 // ---- diagnostics: calc_total_mass / calc_total_energy (diag_mod.F90:10-53) ------

@@ -103,6 +103,8 @@ constexpr int kMxStaging[MX_NVAR] = {kStageLoads, kStageLoads, kStageAsync, kSta
 cudaError_t launch_f64_stage(int var, const F64Stage *d_stages, const WorkItem *d_work, int nwork, int grid,
                              cudaStream_t s);
 int f64_max_grid(int var, int device);
+// the derived metric arrays of MeshF64 (sqrtGf, rsqrtG, lamx, lamy: consecutive fields at out)
+cudaError_t launch_f64_mesh_products(const Layout &L, const MeshF64 &m, double *out, cudaStream_t s);
 
 // central: every stage in d_stages uses a central-difference operator (else WENO-Z);
 // ediss: every stage reconstructs the E-flux dissipation (CCS_EDISS_RECONSTRUCT)
