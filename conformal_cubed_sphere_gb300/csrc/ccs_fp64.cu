@@ -822,7 +822,11 @@ int f64_max_grid(int var, int device) {
 // 61 -> 30; C64, with 96 items, 54 us whole and 58 in parts).  64 x 4 items have no such parts.
 cudaError_t launch_f64_stage(int var, const F64Stage *d_stages, const WorkItem *d_work, int nwork, int grid,
                              cudaStream_t s) {
+#ifdef CCS_BOUNDS
+  const bool split = var != 2 && nwork <= 12;  // (the checked build reaches both on small grids)
+#else
   const bool split = var != 2 && 4 * nwork <= grid;
+#endif
   switch (var) {
     case 1:
       return split ? f64_launch_parts<F64S1>(d_stages, d_work, nwork, s)

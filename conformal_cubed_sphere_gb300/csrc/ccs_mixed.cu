@@ -22,19 +22,22 @@ namespace ccs {
 
 namespace {
 
-// A tile of 32 x TY cells (TY = 32 or 16) and 8 TY threads.  Phase 2 gives each of
-// the TY rows four threads (segments of its 33 x-faces) and each of the 32 columns
-// TY / 8 threads (segments of its TY + 1 y-faces); phase 3 gives each thread four cells.
-template <int TY_>
+// A tile of TX x TY cells.  Phase 2 cuts its rows (TX + 1 x-faces each) and columns (TY
+// + 1 y-faces) into segments of SEG faces (the first SEG + 1), one thread each; phase 3
+// gives each thread SEG / 2 cells.  MINB: resident CTAs an SM the registers are for.
+// PART: a work item consists of several such tiles.
+template <int TX_, int TY_, int SEG_, int MINB_, bool PART_ = false>
 struct MxTile {
-  static constexpr int TX = 32, TY = TY_, NT = 8 * TY;
+  static constexpr int TX = TX_, TY = TY_, SEG = SEG_, MINB = MINB_;
+  static constexpr bool PART = PART_;
+  static constexpr int NTX = TY * (TX / SEG), NT = NTX + TX * (TY / SEG);
   static constexpr int RX = TX + 6, RY = TY + 6;  // halo'd tile
   static constexpr int SP = RX + 1;               // odd pitch: a warp reading one column hits 32 banks
   static constexpr int RN = RY * SP;
   static constexpr int NFL = TX + 1;              // x-faces per tile row
-  static_assert(TY % 8 == 0 && TY <= 32, "column segments of eight faces");
+  static constexpr int CPT = TX * TY / NT;        // cells per thread in phase 3
+  static_assert(TX % SEG == 0 && TY % SEG == 0 && SP % 2 == 1 && CPT * NT == TX * TY, "segments of SEG faces");
 };
-constexpr int SP = 39;  // the smem row pitch, the same for every tile height
 
 // a / b as a times the approximate reciprocal of b (rcp.approx.ftz.f32: one MUFU
 // instruction, a few ulp).  Every denominator here is eps + beta >= eps (at least
@@ -240,6 +243,7 @@ __device__ __forceinline__ void tile_line(SmemMx<T> &S, const MixedStage &st, co
                                           int NFACE, int startg, int lineg) {
   const float phibar = st.phibar, epsF = 4.f * st.eps_F, epsE = 4.f * st.eps_E, epsP = 4.f * st.eps_P;
   const float *__restrict__ Uw = XDIR ? S.u : S.v;  // the wind component along the line
+  constexpr int SP = T::SP;
   const int stp = XDIR ? 1 : SP;
   const int base = XDIR ? (line + 3) * SP + 2 : 2 * SP + line + 3;  // cell ci = 0 of the line
   int o = base + (f0 - 2) * stp;
@@ -347,10 +351,10 @@ __device__ __forceinline__ void tile_line(SmemMx<T> &S, const MixedStage &st, co
 // the line phase, the tendencies and the stage update.
 template <int KIND, class T, bool CENTRAL>
 __device__ __forceinline__ void tile_update(SmemMx<T> &S, const MixedStage &st, const Layout &L, int p, int i0,
-                                            int j0, int lane, int warp) {
-  constexpr int NT = T::NT;
+                                            int j0, int tid) {
+  constexpr int NT = T::NT, TX = T::TX, SP = T::SP, CPT = T::CPT;
   const int N = L.N;
-  // Global operands of phase 3 for this thread's four cells, loaded before the
+  // Global operands of phase 3 for this thread's cells, loaded before the
   // barrier so their latency overlaps the wait for the slowest line segment:
   // f s, 1/s, Y0, the accumulator (or the stage input's hp for RK3) and the
   // compensation terms, as the stage kind needs them.
@@ -358,10 +362,10 @@ __device__ __forceinline__ void tile_update(SmemMx<T> &S, const MixedStage &st, 
   constexpr bool need_acc = kind == K_RK4_2 || kind == K_RK4_4;
   constexpr bool need_in = kind == K_RK3_2 || kind == K_RK3_3;
   constexpr bool need_lo = kind == K_RK4_4 || kind == K_RK3_3;
-  float q_fs[4], q_is[4], q_y0[4][3], q_a[4][3], q_lo[4][3];
+  float q_fs[CPT], q_is[CPT], q_y0[CPT][3], q_a[CPT][3], q_lo[CPT][3];
 #pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int i = i0 + lane, j = j0 + warp + (NT / 32) * k;
+  for (int k = 0; k < CPT; k++) {
+    const int i = i0 + tid % TX, j = j0 + tid / TX + (NT / TX) * k;
     q_fs[k] = q_is[k] = 0.f;
 #pragma unroll
     for (int q = 0; q < 3; q++) q_y0[k][q] = q_a[k][q] = q_lo[k][q] = 0.f;
@@ -380,8 +384,8 @@ __device__ __forceinline__ void tile_update(SmemMx<T> &S, const MixedStage &st, 
 
   // ---- phase 3: tendencies, stage update ---------------------------------------
 #pragma unroll
-  for (int k = 0; k < 4; k++) {
-    const int li = lane, lj = warp + (NT / 32) * k;
+  for (int k = 0; k < CPT; k++) {
+    const int li = tid % TX, lj = tid / TX + (NT / TX) * k;
     const int i = i0 + li, j = j0 + lj;
     if (i > N || j > N) continue;
     const int r = (lj + 3) * SP + li + 3;
@@ -500,20 +504,21 @@ constexpr int kP1Unroll = CCS_MIXED_P1_UNROLL;
 // CENTRAL: the central-difference operators (no face phases); else WENO-Z.
 // STG: the halo-staging schedule of phase 1 (kStageLoads or kStageAsync).
 template <class T, bool CENTRAL, bool EDISS, int STG>
-__global__ void __launch_bounds__(T::NT, CCS_MIXED_MIN_CTAS * 32 / T::TY)
-mixed_stage_kernel(const MixedStage *__restrict__ stages, const WorkItem *__restrict__ work, int nwork) {
-  constexpr int TX = T::TX, TY = T::TY, NT = T::NT, RX = T::RX, RY = T::RY;
-  static_assert(T::SP == SP, "smem pitch");
+__global__ void __launch_bounds__(T::NT, T::MINB)
+mixed_stage_kernel(const MixedStage *__restrict__ stages, const WorkItem *__restrict__ work, int nwork, int sx_,
+                   int sy_) {
+  constexpr int TX = T::TX, TY = T::TY, NT = T::NT, RX = T::RX, RY = T::RY, SP = T::SP, SEG = T::SEG;
   extern __shared__ __align__(16) float smem_f[];
   SmemMx<T> &S = *reinterpret_cast<SmemMx<T> *>(smem_f);
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int tid = threadIdx.x;
+  const int sx = T::PART ? sx_ : 1, sy = T::PART ? sy_ : 1, parts = sx * sy;  // tiles of a work item
 
   constexpr int nwd = (int)(sizeof(MixedStage) / 4);  // descriptor words
   // the first work item's descriptor; each tile then copies the next one into the
   // other buffer asynchronously while it computes
   int buf = 0;
   if (blockIdx.x < nwork) {
-    const WorkItem wi = work[blockIdx.x];
+    const WorkItem wi = work[blockIdx.x / parts];
     const int *src = reinterpret_cast<const int *>(stages + wi.inst);
     int *dst = reinterpret_cast<int *>(&S.stb[0]);
     for (int k = tid; k < nwd; k += NT) dst[k] = src[k];
@@ -524,7 +529,7 @@ mixed_stage_kernel(const MixedStage *__restrict__ stages, const WorkItem *__rest
     const MixedStage &st = S.stb[buf];
     const WorkItem wi = S.wib[buf];
     const int wn = w + gridDim.x;
-    if (tid == 0 && wn < nwork) S.wib[buf ^ 1] = work[wn];  // read by all after the phase-1 barrier
+    if (tid == 0 && wn < nwork) S.wib[buf ^ 1] = work[wn / parts];  // read by all after the phase-1 barrier
 #ifdef CCS_BOUNDS
     {  // poison the tile arrays (checked build only)
       float *a = S.F;
@@ -536,7 +541,8 @@ mixed_stage_kernel(const MixedStage *__restrict__ stages, const WorkItem *__rest
 #endif
     const Layout L = st.L;
     const int N = L.N, p = wi.panel;
-    const int i0 = 1 + wi.tx * TX, j0 = 1 + wi.ty * TY;
+    const int i0 = 1 + (wi.tx * sx + w % sx) * TX, j0 = 1 + (wi.ty * sy + w / sx % sy) * TY;
+    if (T::PART && (i0 > N || j0 > N)) return;  // beyond the panel's edge (a part is its CTA's only tile)
 
     // ---- phase 1: cell quantities on the halo'd tile ------------------------
     if constexpr (STG == kStageAsync) {
@@ -633,14 +639,14 @@ mixed_stage_kernel(const MixedStage *__restrict__ stages, const WorkItem *__rest
     }
     // ---- phase 2: lines -> face values (warps 0-3 rows, 4-7 columns) ---------
     if (!CENTRAL) {  // (the central-difference operators have no faces)
-      // segment seg of a line covers faces 0-8 (seg 0) or 8 seg + 1 .. 8 seg + 8
-      if (tid < 4 * TY) {
+      // segment seg of a line covers faces 0 .. SEG (seg 0) or SEG seg + 1 .. SEG seg + SEG
+      if (tid < T::NTX) {
         const int line = tid % TY, seg = tid / TY;
-        const int f0 = seg == 0 ? 0 : 1 + 8 * seg, nface = seg == 0 ? 9 : 8;
+        const int f0 = seg == 0 ? 0 : 1 + SEG * seg, nface = seg == 0 ? SEG + 1 : SEG;
         if (j0 + line <= N) tile_line<true, EDISS>(S, st, S.F, S.uC, st.m.lamx, L, line, f0, nface, i0 - 1, j0 + line);
       } else {
-        const int t = tid - 4 * TY, line = t % TX, seg = t / TX;
-        const int f0 = seg == 0 ? 0 : 1 + 8 * seg, nface = seg == 0 ? 9 : 8;
+        const int t = tid - T::NTX, line = t % TX, seg = t / TX;
+        const int f0 = seg == 0 ? 0 : 1 + SEG * seg, nface = seg == 0 ? SEG + 1 : SEG;
         if (i0 + line <= N) tile_line<false, EDISS>(S, st, S.G, S.vC, st.m.lamy, L, line, f0, nface, j0 - 1, i0 + line);
       }
     }
@@ -649,13 +655,13 @@ mixed_stage_kernel(const MixedStage *__restrict__ stages, const WorkItem *__rest
     // one stage at a time), so the stage update carries no runtime branches and
     // loads only the operands its kind uses
     switch (st.kind) {
-      case K_RK4_1: tile_update<K_RK4_1, T, CENTRAL>(S, st, L, p, i0, j0, lane, warp); break;
-      case K_RK4_2: tile_update<K_RK4_2, T, CENTRAL>(S, st, L, p, i0, j0, lane, warp); break;
-      case K_RK4_4: tile_update<K_RK4_4, T, CENTRAL>(S, st, L, p, i0, j0, lane, warp); break;
-      case K_RK3_1: tile_update<K_RK3_1, T, CENTRAL>(S, st, L, p, i0, j0, lane, warp); break;
-      case K_RK3_2: tile_update<K_RK3_2, T, CENTRAL>(S, st, L, p, i0, j0, lane, warp); break;
-      case K_RK3_3: tile_update<K_RK3_3, T, CENTRAL>(S, st, L, p, i0, j0, lane, warp); break;
-      default: tile_update<K_TEND, T, CENTRAL>(S, st, L, p, i0, j0, lane, warp); break;
+      case K_RK4_1: tile_update<K_RK4_1, T, CENTRAL>(S, st, L, p, i0, j0, tid); break;
+      case K_RK4_2: tile_update<K_RK4_2, T, CENTRAL>(S, st, L, p, i0, j0, tid); break;
+      case K_RK4_4: tile_update<K_RK4_4, T, CENTRAL>(S, st, L, p, i0, j0, tid); break;
+      case K_RK3_1: tile_update<K_RK3_1, T, CENTRAL>(S, st, L, p, i0, j0, tid); break;
+      case K_RK3_2: tile_update<K_RK3_2, T, CENTRAL>(S, st, L, p, i0, j0, tid); break;
+      case K_RK3_3: tile_update<K_RK3_3, T, CENTRAL>(S, st, L, p, i0, j0, tid); break;
+      default: tile_update<K_TEND, T, CENTRAL>(S, st, L, p, i0, j0, tid); break;
     }
 
     // ---- phase 4: ghost push of the tile's edge strips ----------------------
@@ -817,8 +823,11 @@ __global__ void mixed_diag_kernel(Layout L, StateMixed st, const float *__restri
 
 namespace {
 
-using MxT0 = MxTile<32>;
-using MxT1 = MxTile<16>;
+using MxT0 = MxTile<32, 32, 8, CCS_MIXED_MIN_CTAS>;
+using MxT1 = MxTile<32, 16, 8, 2 * CCS_MIXED_MIN_CTAS>;
+// parts of work items for small launches (see launch_mixed_stage)
+using MxS = MxTile<16, 8, 2, 6, true>;
+using MxM = MxTile<16, 16, 4, 6, true>;
 static_assert(MxT0::TX == kMxTiles[0].tx && MxT0::TY == kMxTiles[0].ty, "tile table");
 static_assert(MxT1::TX == kMxTiles[1].tx && MxT1::TY == kMxTiles[1].ty, "tile table");
 static_assert(MxT0::TX == kMxTiles[2].tx && MxT0::TY == kMxTiles[2].ty, "tile table");
@@ -838,24 +847,27 @@ int mx_grid_for(int device) {  // the WENO instance bounds the occupancy of all
   return sms * per;
 }
 
+// nwork items, each of sx x sy tiles
 template <class T, bool CENTRAL, bool EDISS, int STG>
-cudaError_t mx_launch(const MixedStage *d_stages, const WorkItem *d_work, int nwork, int grid, cudaStream_t s) {
+cudaError_t mx_launch(const MixedStage *d_stages, const WorkItem *d_work, int nwork, int sx, int sy, int grid,
+                      cudaStream_t s) {
   constexpr int smem = (int)sizeof(SmemMx<T>);
   static std::atomic<uint64_t> attr_done{0};
   const cudaError_t e = smem_attr_once((const void *)mixed_stage_kernel<T, CENTRAL, EDISS, STG>, smem, attr_done);
   if (e != cudaSuccess) return e;
-  if (grid > nwork) grid = nwork;
+  const int tiles = nwork * sx * sy;
+  if (grid > tiles) grid = tiles;
   if (grid < 1) return cudaSuccess;
-  mixed_stage_kernel<T, CENTRAL, EDISS, STG><<<grid, T::NT, smem, s>>>(d_stages, d_work, nwork);
+  mixed_stage_kernel<T, CENTRAL, EDISS, STG><<<grid, T::NT, smem, s>>>(d_stages, d_work, tiles, sx, sy);
   return cudaGetLastError();
 }
 
 template <class T, int STG>
 cudaError_t mx_launch_any(bool central, bool ediss, const MixedStage *d_stages, const WorkItem *d_work, int nwork,
-                          int grid, cudaStream_t s) {
-  if (central) return mx_launch<T, true, false, STG>(d_stages, d_work, nwork, grid, s);  // no faces: no E term
-  if (ediss) return mx_launch<T, false, true, STG>(d_stages, d_work, nwork, grid, s);
-  return mx_launch<T, false, false, STG>(d_stages, d_work, nwork, grid, s);
+                          int sx, int sy, int grid, cudaStream_t s) {
+  if (central) return mx_launch<T, true, false, STG>(d_stages, d_work, nwork, sx, sy, grid, s);  // no faces: no E term
+  if (ediss) return mx_launch<T, false, true, STG>(d_stages, d_work, nwork, sx, sy, grid, s);
+  return mx_launch<T, false, false, STG>(d_stages, d_work, nwork, sx, sy, grid, s);
 }
 
 }  // namespace
@@ -869,13 +881,40 @@ int mixed_max_grid(int var, int device) {
   }
 }
 
+// A launch of whole items takes at least the 10 - 12 us that one 32-cell-high tile takes a
+// CTA, alone on its SM: every phase is a chain of loads or of dependent operations.
+// Launches with few items therefore run in smaller tiles with shorter line segments and
+// fewer cells per thread, one CTA each:
+//   16 x 8, two faces a segment, while no SM holds more than three (about C100): C24 11.8
+//   -> 5.7 us a stage, C48 11.8 -> 6.7, C96 11.8 -> 7.7 (C128 10.8, C160 14.7)
+//   16 x 16, four faces a segment, while all of them are resident, six an SM (about C190):
+//   C112 11.8 -> 9.6, C128 11.8 -> 9.7, C160 11.8 -> 10.8, C192 14.0 -> 13.3 (C208 15.4 ->
+//   17.9: the shorter segments compute a quarter more cells, and a second wave begins)
+// Same bits in every tile shape.
 cudaError_t launch_mixed_stage(int var, bool central, bool ediss, const MixedStage *d_stages,
                                const WorkItem *d_work, int nwork, int grid, cudaStream_t s) {
+  const TileShape ts = kMxTiles[var];
+  const int small = nwork * (ts.tx / MxS::TX) * (ts.ty / MxS::TY), mid = nwork * (ts.tx / MxM::TX) * (ts.ty / MxM::TY);
+#ifdef CCS_BOUNDS
+  const int most_small = 6, most_mid = 24;  // (the checked build reaches all three on small grids)
+#else
+  int dev = 0, sms = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
+  const int most_small = 3 * sms, most_mid = 6 * sms;
+#endif
+  if (small <= most_small)
+    return mx_launch_any<MxS, kStageAsync>(central, ediss, d_stages, d_work, nwork, ts.tx / MxS::TX, ts.ty / MxS::TY,
+                                           small, s);
+  if (mid <= most_mid)
+    return mx_launch_any<MxM, kStageLoads>(central, ediss, d_stages, d_work, nwork, ts.tx / MxM::TX, ts.ty / MxM::TY,
+                                           mid, s);
   switch (var) {
-    case 1: return mx_launch_any<MxT1, kStageLoads>(central, ediss, d_stages, d_work, nwork, grid, s);
-    case 2: return mx_launch_any<MxT0, kStageAsync>(central, ediss, d_stages, d_work, nwork, grid, s);
-    case 3: return mx_launch_any<MxT1, kStageAsync>(central, ediss, d_stages, d_work, nwork, grid, s);
-    default: return mx_launch_any<MxT0, kStageLoads>(central, ediss, d_stages, d_work, nwork, grid, s);
+    case 1: return mx_launch_any<MxT1, kStageLoads>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s);
+    case 2: return mx_launch_any<MxT0, kStageAsync>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s);
+    case 3: return mx_launch_any<MxT1, kStageAsync>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s);
+    default: return mx_launch_any<MxT0, kStageLoads>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s);
   }
 }
 
