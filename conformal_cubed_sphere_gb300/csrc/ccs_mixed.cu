@@ -25,9 +25,15 @@ namespace {
 // A tile of TX x TY cells.  Phase 2 cuts its rows (TX + 1 x-faces each) and columns (TY
 // + 1 y-faces) into segments of SEG faces (the first SEG + 1), one thread each; phase 3
 // gives each thread SEG / 2 cells.  MINB: resident CTAs an SM the registers are for.
-// PART: a work item consists of several such tiles.
-template <int TX_, int TY_, int SEG_, int MINB_, bool PART_ = false>
+// PART: a work item consists of several such tiles.  BATCH: cells of the halo'd tile that
+// a thread loads together in phase 1 (kStageLoads), BRANCH: how it skips the others; both
+// as measured: 32 x 32 tiles with five cells (all of a thread's full rows) by branches C384
+// 35.0 -> 33.7 us a stage, C768 150 -> 139 (one cell 35.6 / 150, without the branches 34.9 /
+// 149), 32 x 16 tiles with two without branches C384 35.4 -> 34.9 (six with branches 36.6).
+template <int TX_, int TY_, int SEG_, int MINB_, int BATCH_, bool PART_ = false>
 struct MxTile {
+  static constexpr int BATCH = BATCH_;
+  static constexpr bool BRANCH = TY_ == 32;
   static constexpr int TX = TX_, TY = TY_, SEG = SEG_, MINB = MINB_;
   static constexpr bool PART = PART_;
   static constexpr int NTX = TY * (TX / SEG), NT = NTX + TX * (TY / SEG);
@@ -494,13 +500,6 @@ __device__ __forceinline__ void tile_update(SmemMx<T> &S, const MixedStage &st, 
 #ifndef CCS_MIXED_MIN_CTAS
 #define CCS_MIXED_MIN_CTAS 3
 #endif
-// halo'd-tile cells each thread loads per round in phase 1 (loads in flight); one
-// cell per round measured fastest with three CTAs per SM
-#ifndef CCS_MIXED_P1_UNROLL
-#define CCS_MIXED_P1_UNROLL 1
-#endif
-constexpr int kP1Unroll = CCS_MIXED_P1_UNROLL;
-
 // CENTRAL: the central-difference operators (no face phases); else WENO-Z.
 // STG: the halo-staging schedule of phase 1 (kStageLoads or kStageAsync).
 template <class T, bool CENTRAL, bool EDISS, int STG>
@@ -602,14 +601,16 @@ mixed_stage_kernel(const MixedStage *__restrict__ stages, const WorkItem *__rest
       const float phibar = st.phibar, ha2 = 0.5f * st.a2;
       const float *__restrict__ ihp = st.in.hp, *__restrict__ iu = st.in.u, *__restrict__ iv = st.in.v;
       const MeshMixed m = st.m;
-#pragma unroll kP1Unroll
-      for (int r = tid; r < RX * RY; r += NT) {
-        const int li = r % RX, lj = r / RX;
-        const int i = i0 - 3 + li, j = j0 - 3 + lj;
+      // offsets fit 32 bits: a field has 6 (N + 2 h)^2 cells, N at most 8192
+      const int pan = (int)L.panel * p, origin = (int)L.idx(i0 - 3, j0 - 3, 0), pitch = L.pitch;
+      // A cell that is not there (corner block, beyond the halo) is skipped by a branch
+      // (BRANCH), or reads the panel's first cell and drops it.
+      auto stage = [&](int li, int lj) {  // cell (li, lj) of the halo'd tile
+        const int i = i0 - 3 + li, j = j0 - 3 + lj, a = lj * SP + li;
+        const bool in = i <= N + 3 && j <= N + 3 && !corner(i, j, N);
+        const int cs = T::BRANCH || in ? origin + li + pitch * lj : 0, c = cs + pan;
         float F = 0.f, G = 0.f, E = 0.f, hs = 0.f, sc = 1.f, uC = 0.f, vC = 0.f, u = 0.f, v = 0.f;
-        const int64_t c = L.idx(i, j, p), cs = L.idx(i, j, 0);
-        if (i <= N + 3 && j <= N + 3 && !corner(i, j, N) && ccs_inb(c, L.field, 101) &&
-            ccs_inb(cs, L.panel, 102)) {
+        if ((!T::BRANCH || in) && ccs_inb(c, L.field, 101) && ccs_inb(cs, L.panel, 102)) {
           const float hp = __ldg(ihp + c);
           u = __ldg(iu + c);
           v = __ldg(iv + c);
@@ -623,10 +624,21 @@ mixed_stage_kernel(const MixedStage *__restrict__ stages, const WorkItem *__rest
           hs = __ldg(m.phis + c) + hp;
           E = fmaf(ha2, fmaf(u, uC, v * vC), hs);  // E - phibar
         }
-        const int a = lj * SP + li;
-        if (!ccs_inb(a, T::RN, 103)) continue;
-        S.F[a] = F; S.G[a] = G; S.E[a] = E; S.hs[a] = hs; S.s[a] = sc;
-        S.uC[a] = uC; S.vC[a] = vC; S.u[a] = u; S.v[a] = v;
+        if (!ccs_inb(a, T::RN, 103)) return;
+        const bool ok = T::BRANCH || in;
+        S.F[a] = ok ? F : 0.f; S.G[a] = ok ? G : 0.f; S.E[a] = ok ? E : 0.f; S.hs[a] = ok ? hs : 0.f;
+        S.s[a] = ok ? sc : 1.f; S.uC[a] = ok ? uC : 0.f; S.vC[a] = ok ? vC : 0.f; S.u[a] = ok ? u : 0.f;
+        S.v[a] = ok ? v : 0.f;
+      };
+      if constexpr (TX == 32) {
+        // a warp takes a row's first 32 cells, the rows NT / 32 apart; the last six cells
+        // of all rows are dealt out to the threads: no division per cell
+#pragma unroll T::BATCH
+        for (int lj = tid >> 5; lj < RY; lj += NT / 32) stage(tid & 31, lj);
+        for (int r = tid; r < (RX - 32) * RY; r += NT) stage(32 + r % (RX - 32), r / (RX - 32));
+      } else {
+#pragma unroll T::BATCH
+        for (int r = tid; r < RX * RY; r += NT) stage(r % RX, r / RX);
       }
     }
     __syncthreads();
@@ -823,11 +835,11 @@ __global__ void mixed_diag_kernel(Layout L, StateMixed st, const float *__restri
 
 namespace {
 
-using MxT0 = MxTile<32, 32, 8, CCS_MIXED_MIN_CTAS>;
-using MxT1 = MxTile<32, 16, 8, 2 * CCS_MIXED_MIN_CTAS>;
+using MxT0 = MxTile<32, 32, 8, CCS_MIXED_MIN_CTAS, 5>;
+using MxT1 = MxTile<32, 16, 8, 2 * CCS_MIXED_MIN_CTAS, 2>;
 // parts of work items for small launches (see launch_mixed_stage)
-using MxS = MxTile<16, 8, 2, 6, true>;
-using MxM = MxTile<16, 16, 4, 6, true>;
+using MxS = MxTile<16, 8, 2, 6, 1, true>;
+using MxM = MxTile<16, 16, 4, 6, 3, true>;
 static_assert(MxT0::TX == kMxTiles[0].tx && MxT0::TY == kMxTiles[0].ty, "tile table");
 static_assert(MxT1::TX == kMxTiles[1].tx && MxT1::TY == kMxTiles[1].ty, "tile table");
 static_assert(MxT0::TX == kMxTiles[2].tx && MxT0::TY == kMxTiles[2].ty, "tile table");
