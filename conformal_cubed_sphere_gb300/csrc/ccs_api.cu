@@ -400,7 +400,7 @@ static int f64_enqueue_step(ccs_handle *h, bool with_sw) {
   for (int k = 0; k < h->n_rk; k++) {
     const F64Stage *d = h->d_stages + ((k == h->n_rk - 1 && with_sw) ? h->n_rk : k);
     if (h->timing) CCS_TRY(h, cudaEventRecord(h->ev0, h->stream));
-    CCS_TRY(h, launch_f64_stage(h->var, d, h->d_work, h->nwork, h->grid, h->stream));
+    CCS_TRY(h, launch_f64_stage(h->var, d, h->d_work, h->nwork, h->grid, h->stream, k > 0 && !h->timing));
     if (h->timing) {
       CCS_TRY(h, cudaEventRecord(h->ev1, h->stream));
       CCS_TRY(h, cudaEventSynchronize(h->ev1));
@@ -1101,10 +1101,10 @@ static bool mixed_has_stages(const ccs_handle *h) { return h->mixed->have_phibar
 
 // one launch of the handle's mixed stage kernel instance (tile variant, operator
 // family, E-flux option) over stage descriptor d
-static cudaError_t mixed_launch(ccs_handle *h, const MixedStage *d) {
+static cudaError_t mixed_launch(ccs_handle *h, const MixedStage *d, bool chained = false) {
   MixedLane *M = h->mixed;
   return launch_mixed_stage(M->var, h->op != CCS_OP_WENO, h->cfg.e_dissipation != CCS_EDISS_ZERO, d, M->d_work,
-                            M->nwork, M->grid, h->stream);
+                            M->nwork, M->grid, h->stream, chained);
 }
 
 static int mixed_sync(ccs_handle *h) {
@@ -1118,7 +1118,7 @@ static int mixed_enqueue_step(ccs_handle *h) {
   MixedLane *M = h->mixed;
   for (int k = 0; k < M->n_rk; k++) {
     if (h->timing) CCS_TRY(h, cudaEventRecord(h->ev0, h->stream));
-    CCS_TRY(h, mixed_launch(h, M->d_stages + k));
+    CCS_TRY(h, mixed_launch(h, M->d_stages + k, k > 0 && !h->timing));
     if (h->timing) {
       CCS_TRY(h, cudaEventRecord(h->ev1, h->stream));
       CCS_TRY(h, cudaEventSynchronize(h->ev1));
@@ -1414,14 +1414,14 @@ static int group_nvar(const BatchGroup &g) { return g.lane == CCS_FP64 ? F64_NVA
 
 // Stage k of group g (k = n_rk - 1 with with_sw: the FP64 final stage that also
 // writes the sphere winds) as one launch over the work list of all its members.
-static cudaError_t group_launch(BatchGroup &g, int k, bool with_sw) {
+static cudaError_t group_launch(BatchGroup &g, int k, bool with_sw, bool chained = false) {
   if (g.lane == CCS_FP64) {
     const int row = (k == g.n_rk - 1 && with_sw) ? g.n_rk : k;
     return launch_f64_stage(g.var, (const F64Stage *)g.d_stages + (size_t)row * g.nmem, g.d_work, g.nwork, g.grid,
-                            g.stream);
+                            g.stream, chained);
   }
   return launch_mixed_stage(g.var, g.central, g.ediss, (const MixedStage *)g.d_stages + (size_t)k * g.nmem,
-                            g.d_work, g.nwork, g.grid, g.stream);
+                            g.d_work, g.nwork, g.grid, g.stream, chained);
 }
 
 // (Re)builds group g's work list for tile variant var: every tile of the six panels
@@ -1458,7 +1458,7 @@ static int batch_enqueue(ccs_batch *b, bool with_sw) {
   BATCH_TRY(b, cudaEventRecord(b->fork, b->stream));
   for (auto &g : b->groups) {
     BATCH_TRY(b, cudaStreamWaitEvent(g.stream, b->fork, 0));
-    for (int k = 0; k < g.n_rk; k++) BATCH_TRY(b, group_launch(g, k, with_sw));
+    for (int k = 0; k < g.n_rk; k++) BATCH_TRY(b, group_launch(g, k, with_sw, k > 0));
     BATCH_TRY(b, cudaEventRecord(g.done, g.stream));
     BATCH_TRY(b, cudaStreamWaitEvent(b->stream, g.done, 0));
   }

@@ -532,6 +532,8 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
     __syncthreads();
 #endif
 
+    stage_wait();
+
     // ---- phase 1: cell quantities (spatial_operators_mod.F90:71-78) ----------
     // (cells outside the panel and its edge halos are set to zero: the faces that
     // would read them belong to no interior cell)
@@ -542,11 +544,11 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
       double phit = 0., phitG = 0., E = 0., Fx = 0., Fy = 0., uC = 0., vC = 0., u = 0., v = 0.;
       const int64_t c = L.idx(i, j, p);
       if (i >= -2 && i <= N + 3 && j >= -2 && j <= N + 3 && !is_corner(i, j, N) && ccs_inb(c, L.field, 201)) {
-        const double phiG = __ldg(st.in.phiG + c), phi = __ldg(st.in.phi + c);
-        u = __ldg(st.in.u + c);
-        v = __ldg(st.in.v + c);
-        uC = __ldg(st.in.uC + c);
-        vC = __ldg(st.in.vC + c);
+        const double phiG = __ldcg(st.in.phiG + c), phi = __ldcg(st.in.phi + c);
+        u = __ldcg(st.in.u + c);
+        v = __ldcg(st.in.v + c);
+        uC = __ldcg(st.in.uC + c);
+        vC = __ldcg(st.in.vC + c);
         phit = f.add(phi, __ldg(st.m.phis + c));
         phitG = f.mul(phit, __ldg(st.m.sqrtG + c));
         const double K = half_of(f.add(f.mul(u, uC), f.mul(v, vC)));
@@ -628,9 +630,9 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
         const double sgf = __ldg(st.m.sqrtGf + c);
         double y0[3] = {0., 0., 0.}, ac[3] = {0., 0., 0.};
         if (kind != K_TEND) {
-          y0[0] = st.y0phiG[c]; y0[1] = st.y0u[c]; y0[2] = st.y0v[c];
-          if (kind == K_RK4_2 || kind == K_RK4_4) { ac[0] = st.accphiG[c]; ac[1] = st.accu[c]; ac[2] = st.accv[c]; }
-          if (kind == K_RK3_2 || kind == K_RK3_3) { ac[0] = __ldg(st.in.phiG + c); ac[1] = S.u[rc]; ac[2] = S.v[rc]; }
+          y0[0] = __ldcg(st.y0phiG + c); y0[1] = __ldcg(st.y0u + c); y0[2] = __ldcg(st.y0v + c);
+          if (kind == K_RK4_2 || kind == K_RK4_4) { ac[0] = __ldcg(st.accphiG + c); ac[1] = __ldcg(st.accu + c); ac[2] = __ldcg(st.accv + c); }
+          if (kind == K_RK3_2 || kind == K_RK3_3) { ac[0] = __ldcg(st.in.phiG + c); ac[1] = S.u[rc]; ac[2] = S.v[rc]; }
         }
         const double a11 = __ldg(st.m.aig11 + c), a12 = __ldg(st.m.aig12 + c), a21 = __ldg(st.m.aig21 + c),
                      a22 = __ldg(st.m.aig22 + c);
@@ -693,6 +695,7 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
     }
     __syncthreads();
 
+    if (w + gridDim.x >= nwork) stage_release();  // this CTA's last item is all but done
     // ---- phase 4: ghost push of the part's edge strips ------------------------
     // A cell within `halo` of a panel edge lands in that edge's halo strip (two strips
     // near a panel corner).  The strip cells of the part, strip by strip (0 left, 1
@@ -784,22 +787,26 @@ int f64_grid_for(int device) {
 }
 
 template <class T>
-cudaError_t f64_launch(const F64Stage *d_stages, const WorkItem *d_work, int nwork, int grid, cudaStream_t s) {
+cudaError_t f64_launch(const F64Stage *d_stages, const WorkItem *d_work, int nwork, int grid, cudaStream_t s,
+                       bool chained) {
   constexpr int smem = f64_smem_bytes<T>();
   static std::atomic<uint64_t> attr_done{0};
   const cudaError_t e = smem_attr_once((const void *)f64_stage_kernel<T>, smem, attr_done);
   if (e != cudaSuccess) return e;
   if (grid > nwork) grid = nwork;
   if (grid < 1) return cudaSuccess;
-  f64_stage_kernel<T><<<grid, T::NT, smem, s>>>(d_stages, d_work, nwork);
-  return cudaGetLastError();
+  // chained only with one item a CTA: CTAs that start early spread unevenly over the SMs,
+  // which costs more than it saves when some have an item more than others (C384: 921 us a
+  // stage unchained, 933 chained; C24 23.6 -> 23.1, C48 30.1 -> 29.5)
+  return launch_stage(f64_stage_kernel<T>, grid, T::NT, smem, s, chained && grid == nwork, d_stages, d_work, nwork);
 }
 
 // the same work items in parts, one CTA each
 template <class T>
-cudaError_t f64_launch_parts(const F64Stage *d_stages, const WorkItem *d_work, int nwork, cudaStream_t s) {
+cudaError_t f64_launch_parts(const F64Stage *d_stages, const WorkItem *d_work, int nwork, cudaStream_t s,
+                             bool chained) {
   const int parts = nwork * T::SX * T::SY;
-  return f64_launch<T>(d_stages, d_work, parts, parts, s);
+  return f64_launch<T>(d_stages, d_work, parts, parts, s, chained);
 }
 
 static_assert(F64T0::TX == kF64Tiles[0].tx && F64T0::TY == kF64Tiles[0].ty, "tile table");
@@ -821,7 +828,7 @@ int f64_max_grid(int var, int device) {
 // cells 24 us on an SM of their own and 30 us two to an SM (C24: 61 -> 24 us a stage, C48
 // 61 -> 30; C64, with 96 items, 54 us whole and 58 in parts).  64 x 4 items have no such parts.
 cudaError_t launch_f64_stage(int var, const F64Stage *d_stages, const WorkItem *d_work, int nwork, int grid,
-                             cudaStream_t s) {
+                             cudaStream_t s, bool chained) {
 #ifdef CCS_BOUNDS
   const bool split = var != 2 && nwork <= 12;  // (the checked build reaches both on small grids)
 #else
@@ -829,12 +836,12 @@ cudaError_t launch_f64_stage(int var, const F64Stage *d_stages, const WorkItem *
 #endif
   switch (var) {
     case 1:
-      return split ? f64_launch_parts<F64S1>(d_stages, d_work, nwork, s)
-                   : f64_launch<F64T1>(d_stages, d_work, nwork, grid, s);
-    case 2: return f64_launch<F64T2>(d_stages, d_work, nwork, grid, s);
+      return split ? f64_launch_parts<F64S1>(d_stages, d_work, nwork, s, chained)
+                   : f64_launch<F64T1>(d_stages, d_work, nwork, grid, s, chained);
+    case 2: return f64_launch<F64T2>(d_stages, d_work, nwork, grid, s, chained);
     default:
-      return split ? f64_launch_parts<F64S0>(d_stages, d_work, nwork, s)
-                   : f64_launch<F64T0>(d_stages, d_work, nwork, grid, s);
+      return split ? f64_launch_parts<F64S0>(d_stages, d_work, nwork, s, chained)
+                   : f64_launch<F64T0>(d_stages, d_work, nwork, grid, s, chained);
   }
 }
 

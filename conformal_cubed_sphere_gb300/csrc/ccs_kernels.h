@@ -26,6 +26,36 @@ inline cudaError_t smem_attr_once(const void *fn, int smem, std::atomic<uint64_t
   return e;
 }
 
+// Launches a stage kernel.  chained: the launch before it in the stream is the same
+// step's previous stage, whose end the kernel itself waits for (stage_wait): its CTAs may
+// start, and read their work items and descriptors, while that stage drains.
+template <class... P, class... A>
+cudaError_t launch_stage(void (*kernel)(P...), int grid, int block, int smem, cudaStream_t s, bool chained,
+                         A... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = dim3((unsigned)grid);
+  cfg.blockDim = dim3((unsigned)block);
+  cfg.dynamicSmemBytes = (size_t)smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = chained ? 1 : 0;
+  return cudaLaunchKernelEx(&cfg, kernel, static_cast<P>(args)...);
+}
+
+#if defined(__CUDACC__)
+// lets the next chained stage start its CTAs where they fit, called as a CTA's last tile
+// nears its end (at the kernel's start it crowds the next stage's CTAs onto the SMs that
+// have room: mixed C150 10.3 -> 12.0 us a stage)
+__device__ __forceinline__ void stage_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+// waits until the previous stage of a chained launch has ended and its writes are visible
+// (returns at once in other launches).  Whatever a stage writes is read after this and
+// through L2 (__ldcg): this SM's L1 may hold lines that the previous stage read.
+__device__ __forceinline__ void stage_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+#endif
+
 // One tile of work: instance, panel (0..5) and tile coordinates.
 struct WorkItem {
   int16_t inst, panel, tx, ty;
@@ -101,7 +131,7 @@ constexpr int kMxStaging[MX_NVAR] = {kStageLoads, kStageLoads, kStageAsync, kSta
 
 // kernel launchers (return cudaGetLastError()); `var` indexes the tile tables
 cudaError_t launch_f64_stage(int var, const F64Stage *d_stages, const WorkItem *d_work, int nwork, int grid,
-                             cudaStream_t s);
+                             cudaStream_t s, bool chained = false);
 int f64_max_grid(int var, int device);
 // the derived metric arrays of MeshF64 (sqrtGf, rsqrtG, lamx, lamy: consecutive fields at out)
 cudaError_t launch_f64_mesh_products(const Layout &L, const MeshF64 &m, double *out, cudaStream_t s);
@@ -109,7 +139,8 @@ cudaError_t launch_f64_mesh_products(const Layout &L, const MeshF64 &m, double *
 // central: every stage in d_stages uses a central-difference operator (else WENO-Z);
 // ediss: every stage reconstructs the E-flux dissipation (CCS_EDISS_RECONSTRUCT)
 cudaError_t launch_mixed_stage(int var, bool central, bool ediss, const MixedStage *d_stages,
-                               const WorkItem *d_work, int nwork, int grid, cudaStream_t s);
+                               const WorkItem *d_work, int nwork, int grid, cudaStream_t s,
+                               bool chained = false);
 int mixed_max_grid(int var, int device);
 cudaError_t launch_mixed_import(const Layout &L, const double *phi, const double *u, const double *v,
                                 double phibar, double inv_a2, StateMixed out, float *lohp, float *lou,

@@ -381,10 +381,10 @@ __device__ __forceinline__ void tile_update(SmemMx<T> &S, const MixedStage &st, 
     q_fs[k] = __ldg(st.m.fs + c);
     q_is[k] = __ldg(st.m.inv_s + L.idx(i, j, 0));
     if constexpr (kind == K_TEND) continue;
-    q_y0[k][0] = st.y0hp[c]; q_y0[k][1] = st.y0u[c]; q_y0[k][2] = st.y0v[c];
-    if (need_acc) { q_a[k][0] = st.acchp[c]; q_a[k][1] = st.accu[c]; q_a[k][2] = st.accv[c]; }
-    if (need_in) q_a[k][0] = st.in.hp[c];
-    if (need_lo) { q_lo[k][0] = st.lohp[c]; q_lo[k][1] = st.lou[c]; q_lo[k][2] = st.lov[c]; }
+    q_y0[k][0] = __ldcg(st.y0hp + c); q_y0[k][1] = __ldcg(st.y0u + c); q_y0[k][2] = __ldcg(st.y0v + c);
+    if (need_acc) { q_a[k][0] = __ldcg(st.acchp + c); q_a[k][1] = __ldcg(st.accu + c); q_a[k][2] = __ldcg(st.accv + c); }
+    if (need_in) q_a[k][0] = __ldcg(st.in.hp + c);
+    if (need_lo) { q_lo[k][0] = __ldcg(st.lohp + c); q_lo[k][1] = __ldcg(st.lou + c); q_lo[k][2] = __ldcg(st.lov + c); }
   }
   __syncthreads();
 
@@ -524,6 +524,7 @@ mixed_stage_kernel(const MixedStage *__restrict__ stages, const WorkItem *__rest
     if (tid == 0) S.wib[0] = wi;
   }
   __syncthreads();
+  stage_wait();
   for (int w = blockIdx.x; w < nwork; w += gridDim.x, buf ^= 1) {
     const MixedStage &st = S.stb[buf];
     const WorkItem wi = S.wib[buf];
@@ -550,7 +551,7 @@ mixed_stage_kernel(const MixedStage *__restrict__ stages, const WorkItem *__rest
       // registers; after its own copies land, the thread turns each of its cells
       // into the cell quantities in place
       const float phibar = st.phibar, ha2 = 0.5f * st.a2;
-      const float *__restrict__ ihp = st.in.hp, *__restrict__ iu = st.in.u, *__restrict__ iv = st.in.v;
+      const float *ihp = st.in.hp, *iu = st.in.u, *iv = st.in.v;
       const MeshMixed m = st.m;
       for (int r = tid; r < RX * RY; r += NT) {
         const int li = r % RX, lj = r / RX;
@@ -599,7 +600,7 @@ mixed_stage_kernel(const MixedStage *__restrict__ stages, const WorkItem *__rest
       // each thread loads its cells' raw inputs into registers (coalesced rows of the
       // halo'd tile) and stores the derived cell quantities
       const float phibar = st.phibar, ha2 = 0.5f * st.a2;
-      const float *__restrict__ ihp = st.in.hp, *__restrict__ iu = st.in.u, *__restrict__ iv = st.in.v;
+      const float *ihp = st.in.hp, *iu = st.in.u, *iv = st.in.v;
       const MeshMixed m = st.m;
       // offsets fit 32 bits: a field has 6 (N + 2 h)^2 cells, N at most 8192
       const int pan = (int)L.panel * p, origin = (int)L.idx(i0 - 3, j0 - 3, 0), pitch = L.pitch;
@@ -611,9 +612,9 @@ mixed_stage_kernel(const MixedStage *__restrict__ stages, const WorkItem *__rest
         const int cs = T::BRANCH || in ? origin + li + pitch * lj : 0, c = cs + pan;
         float F = 0.f, G = 0.f, E = 0.f, hs = 0.f, sc = 1.f, uC = 0.f, vC = 0.f, u = 0.f, v = 0.f;
         if ((!T::BRANCH || in) && ccs_inb(c, L.field, 101) && ccs_inb(cs, L.panel, 102)) {
-          const float hp = __ldg(ihp + c);
-          u = __ldg(iu + c);
-          v = __ldg(iv + c);
+          const float hp = __ldcg(ihp + c);
+          u = __ldcg(iu + c);
+          v = __ldcg(iv + c);
           sc = __ldg(m.s + cs);
           const float4 g = __ldg(m.ig + cs);
           uC = fmaf(g.x, u, g.y * v);
@@ -676,6 +677,7 @@ mixed_stage_kernel(const MixedStage *__restrict__ stages, const WorkItem *__rest
       default: tile_update<K_TEND, T, CENTRAL>(S, st, L, p, i0, j0, tid); break;
     }
 
+    if (wn >= nwork) stage_release();  // this CTA's last tile is all but done
     // ---- phase 4: ghost push of the tile's edge strips ----------------------
     // hp copies; the covariant wind crosses the edge through the FP64 2x2
     // transform G_h IA_h A_s IG_s of the receiving halo cell.  Entries are dealt
@@ -862,7 +864,7 @@ int mx_grid_for(int device) {  // the WENO instance bounds the occupancy of all
 // nwork items, each of sx x sy tiles
 template <class T, bool CENTRAL, bool EDISS, int STG>
 cudaError_t mx_launch(const MixedStage *d_stages, const WorkItem *d_work, int nwork, int sx, int sy, int grid,
-                      cudaStream_t s) {
+                      cudaStream_t s, bool chained) {
   constexpr int smem = (int)sizeof(SmemMx<T>);
   static std::atomic<uint64_t> attr_done{0};
   const cudaError_t e = smem_attr_once((const void *)mixed_stage_kernel<T, CENTRAL, EDISS, STG>, smem, attr_done);
@@ -870,16 +872,16 @@ cudaError_t mx_launch(const MixedStage *d_stages, const WorkItem *d_work, int nw
   const int tiles = nwork * sx * sy;
   if (grid > tiles) grid = tiles;
   if (grid < 1) return cudaSuccess;
-  mixed_stage_kernel<T, CENTRAL, EDISS, STG><<<grid, T::NT, smem, s>>>(d_stages, d_work, tiles, sx, sy);
-  return cudaGetLastError();
+  return launch_stage(mixed_stage_kernel<T, CENTRAL, EDISS, STG>, grid, T::NT, smem, s, chained, d_stages, d_work,
+                      tiles, sx, sy);
 }
 
 template <class T, int STG>
 cudaError_t mx_launch_any(bool central, bool ediss, const MixedStage *d_stages, const WorkItem *d_work, int nwork,
-                          int sx, int sy, int grid, cudaStream_t s) {
-  if (central) return mx_launch<T, true, false, STG>(d_stages, d_work, nwork, sx, sy, grid, s);  // no faces: no E term
-  if (ediss) return mx_launch<T, false, true, STG>(d_stages, d_work, nwork, sx, sy, grid, s);
-  return mx_launch<T, false, false, STG>(d_stages, d_work, nwork, sx, sy, grid, s);
+                          int sx, int sy, int grid, cudaStream_t s, bool chained) {
+  if (central) return mx_launch<T, true, false, STG>(d_stages, d_work, nwork, sx, sy, grid, s, chained);  // no faces: no E term
+  if (ediss) return mx_launch<T, false, true, STG>(d_stages, d_work, nwork, sx, sy, grid, s, chained);
+  return mx_launch<T, false, false, STG>(d_stages, d_work, nwork, sx, sy, grid, s, chained);
 }
 
 }  // namespace
@@ -904,7 +906,8 @@ int mixed_max_grid(int var, int device) {
 //   17.9: the shorter segments compute a quarter more cells, and a second wave begins)
 // Same bits in every tile shape.
 cudaError_t launch_mixed_stage(int var, bool central, bool ediss, const MixedStage *d_stages,
-                               const WorkItem *d_work, int nwork, int grid, cudaStream_t s) {
+                               const WorkItem *d_work, int nwork, int grid, cudaStream_t s,
+                               bool chained) {
   const TileShape ts = kMxTiles[var];
   const int small = nwork * (ts.tx / MxS::TX) * (ts.ty / MxS::TY), mid = nwork * (ts.tx / MxM::TX) * (ts.ty / MxM::TY);
 #ifdef CCS_BOUNDS
@@ -918,15 +921,15 @@ cudaError_t launch_mixed_stage(int var, bool central, bool ediss, const MixedSta
 #endif
   if (small <= most_small)
     return mx_launch_any<MxS, kStageAsync>(central, ediss, d_stages, d_work, nwork, ts.tx / MxS::TX, ts.ty / MxS::TY,
-                                           small, s);
+                                           small, s, chained);
   if (mid <= most_mid)
     return mx_launch_any<MxM, kStageLoads>(central, ediss, d_stages, d_work, nwork, ts.tx / MxM::TX, ts.ty / MxM::TY,
-                                           mid, s);
+                                           mid, s, chained);
   switch (var) {
-    case 1: return mx_launch_any<MxT1, kStageLoads>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s);
-    case 2: return mx_launch_any<MxT0, kStageAsync>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s);
-    case 3: return mx_launch_any<MxT1, kStageAsync>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s);
-    default: return mx_launch_any<MxT0, kStageLoads>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s);
+    case 1: return mx_launch_any<MxT1, kStageLoads>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s, chained);
+    case 2: return mx_launch_any<MxT0, kStageAsync>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s, chained);
+    case 3: return mx_launch_any<MxT1, kStageAsync>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s, chained);
+    default: return mx_launch_any<MxT0, kStageLoads>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s, chained);
   }
 }
 
