@@ -166,20 +166,28 @@ struct ccs_handle {
 
 static const int kDiagBlocks = 512;
 
-static int upload_field(ccs_handle *h, double *dst, const double *src) {
-  const Layout &L = h->L;
-  CCS_TRY(h, cudaMemcpy2DAsync(dst, (size_t)L.pitch * sizeof(double), src, (size_t)L.nh * sizeof(double),
-                               (size_t)L.nh * sizeof(double), (size_t)L.nh * 6, cudaMemcpyHostToDevice,
-                               h->stream));
-  return CCS_OK;
-}
-
-static int download_field(ccs_handle *h, double *dst, const double *src) {
-  const Layout &L = h->L;
-  CCS_TRY(h, cudaMemcpy2DAsync(dst, (size_t)L.nh * sizeof(double), src, (size_t)L.pitch * sizeof(double),
-                               (size_t)L.nh * sizeof(double), (size_t)L.nh * 6, cudaMemcpyDeviceToHost,
-                               h->stream));
-  return CCS_OK;
+// Copies n fields of `bytes` each (dst[q] <- src[q], NULL entries skipped), one
+// cudaMemcpyAsync per run of fields whose destination and source both continue the
+// previous field's: a caller whose host arrays are consecutive slices of one
+// page-locked block gets one copy per direction, which the host link overlaps
+// with the other direction better than many smaller copies.
+static cudaError_t copy_field_runs(void *const *dst, const void *const *src, int n, size_t bytes,
+                                   cudaMemcpyKind kind, cudaStream_t s) {
+  int q = 0;
+  while (q < n) {
+    if (!dst[q] || !src[q]) {
+      q++;
+      continue;
+    }
+    int e = q + 1;
+    while (e < n && dst[e] && src[e] && (char *)dst[e] == (char *)dst[e - 1] + bytes &&
+           (const char *)src[e] == (const char *)src[e - 1] + bytes)
+      e++;
+    const cudaError_t err = cudaMemcpyAsync(dst[q], src[q], (size_t)(e - q) * bytes, kind, s);
+    if (err != cudaSuccess) return err;
+    q = e;
+  }
+  return cudaSuccess;
 }
 
 static int validate_config(const ccs_config *c) {
@@ -273,11 +281,13 @@ static int build_mesh(ccs_handle *h, const ccs_mesh_view *mv) {
     matmul22(&mv->matrixG[4 * c], &mv->matrixIA[4 * c], M);  // projection_mod.F90:71
     t[11][c] = M[0]; t[12][c] = M[2]; t[13][c] = M[1]; t[14][c] = M[3];
   }
-  for (int k = 0; k < na; k++) {
-    int rc = upload_field(h, dm->buf64 + k * nf, t[k]);
-    if (rc) return rc;
-  }
   double *b = dm->buf64;
+  if (L.pitch == L.nh)
+    CCS_TRY(h, cudaMemcpyAsync(b, tmp.data(), na * nf * sizeof(double), cudaMemcpyHostToDevice, h->stream));
+  else
+    CCS_TRY(h, cudaMemcpy2DAsync(b, (size_t)L.pitch * sizeof(double), tmp.data(), (size_t)L.nh * sizeof(double),
+                                 (size_t)L.nh * sizeof(double), (size_t)L.nh * 6 * na, cudaMemcpyHostToDevice,
+                                 h->stream));
   dm->m64.sqrtG = b + 0 * nf; dm->m64.phis = b + 1 * nf; dm->m64.f = b + 2 * nf;
   dm->m64.ig11 = b + 3 * nf; dm->m64.ig12 = b + 4 * nf; dm->m64.ig21 = b + 5 * nf; dm->m64.ig22 = b + 6 * nf;
   dm->m64.aig11 = b + 7 * nf; dm->m64.aig12 = b + 8 * nf; dm->m64.aig21 = b + 9 * nf; dm->m64.aig22 = b + 10 * nf;
@@ -540,7 +550,9 @@ static int init_common(const ccs_config *cfg, ccs_handle **out, ccs_handle **hp)
   ccs_handle *h = new ccs_handle();
   h->cfg = *cfg;
   const int nh = cfg->N + 2 * cfg->halo;
-  h->L = make_layout(cfg->N, cfg->halo, round_up(nh, 4));
+  // the FP64 lane keeps the reference's rows, so that a host field is one contiguous copy
+  // (its kernels are bound by arithmetic); the mixed lane pads them for 16-byte loads
+  h->L = make_layout(cfg->N, cfg->halo, cfg->precision == CCS_FP64 ? nh : round_up(nh, 4));
   if (cudaStreamCreateWithFlags(&h->stream, cudaStreamNonBlocking) != cudaSuccess) {
     delete h;
     return CCS_ERR_CUDA;
@@ -622,19 +634,13 @@ static int set_state_impl(ccs_handle *h, const ccs_state_view *s, bool sync) {
   if (!h || !s || !s->phiG || !s->u || !s->v || !s->phi || !s->uC || !s->vC) return CCS_ERR_ARG;
   cudaSetDevice(h->cfg.device);
   if (h->cfg.precision == CCS_MIXED) return mixed_set_state(h, s, sync);
-  const double *src[6] = {s->phiG, s->u, s->v, s->phi, s->uC, s->vC};
-  double *dst[6] = {h->S[0].phiG, h->S[0].u, h->S[0].v, h->S[0].phi, h->S[0].uC, h->S[0].vC};
-  for (int k = 0; k < 6; k++) {
-    int rc = upload_field(h, dst[k], src[k]);
-    if (rc) return rc;
-  }
-  h->sphere_valid = false;
-  if (s->zonal_wind && s->meridional_wind) {
-    int rc = upload_field(h, h->zonal, s->zonal_wind);
-    if (!rc) rc = upload_field(h, h->merid, s->meridional_wind);
-    if (rc) return rc;
-    h->sphere_valid = true;
-  }
+  const StateF64 &S = h->S[0];
+  const bool sphere = s->zonal_wind && s->meridional_wind;
+  void *const dst[8] = {S.phiG, S.u, S.v, S.phi, S.uC, S.vC, h->zonal, h->merid};
+  const void *const src[8] = {s->phiG, s->u, s->v, s->phi, s->uC, s->vC, s->zonal_wind, s->meridional_wind};
+  CCS_TRY(h, copy_field_runs(dst, src, sphere ? 8 : 6, (size_t)h->L.field * sizeof(double), cudaMemcpyHostToDevice,
+                             h->stream));
+  h->sphere_valid = sphere;
   if (sync) CCS_TRY(h, cudaStreamSynchronize(h->stream));
   return CCS_OK;
 }
@@ -647,23 +653,11 @@ static int get_state_impl(ccs_handle *h, ccs_state_view *s, bool sync) {
   if (!h || !s) return CCS_ERR_ARG;
   cudaSetDevice(h->cfg.device);
   if (h->cfg.precision == CCS_MIXED) return mixed_get_state(h, s, sync);
-  double *dst[6] = {s->phiG, s->u, s->v, s->phi, s->uC, s->vC};
-  const double *src[6] = {h->S[0].phiG, h->S[0].u, h->S[0].v, h->S[0].phi, h->S[0].uC, h->S[0].vC};
-  for (int k = 0; k < 6; k++)
-    if (dst[k]) {
-      int rc = download_field(h, dst[k], src[k]);
-      if (rc) return rc;
-    }
-  if (h->sphere_valid) {
-    if (s->zonal_wind) {
-      int rc = download_field(h, s->zonal_wind, h->zonal);
-      if (rc) return rc;
-    }
-    if (s->meridional_wind) {
-      int rc = download_field(h, s->meridional_wind, h->merid);
-      if (rc) return rc;
-    }
-  }
+  const StateF64 &S = h->S[0];
+  void *const dst[8] = {s->phiG, s->u, s->v, s->phi, s->uC, s->vC, s->zonal_wind, s->meridional_wind};
+  const void *const src[8] = {S.phiG, S.u, S.v, S.phi, S.uC, S.vC, h->zonal, h->merid};
+  CCS_TRY(h, copy_field_runs(dst, src, h->sphere_valid ? 8 : 6, (size_t)h->L.field * sizeof(double),
+                             cudaMemcpyDeviceToHost, h->stream));
   if (sync) CCS_TRY(h, cudaStreamSynchronize(h->stream));
   return CCS_OK;
 }
@@ -720,12 +714,9 @@ int ccs_spatial_operator(ccs_handle *h, double *tp, double *tu, double *tv) {
   if (h->cfg.precision == CCS_MIXED) return mixed_tend(h, tp, tu, tv);
   const F64Stage *d = h->d_stages + h->n_rk + 1;
   CCS_TRY(h, launch_f64_stage(h->var, d, h->d_work, h->nwork, h->grid, h->stream));
-  double *dst[3] = {tp, tu, tv};
-  for (int k = 0; k < 3; k++)
-    if (dst[k]) {
-      int rc = download_field(h, dst[k], h->tend[k]);
-      if (rc) return rc;
-    }
+  void *const dst[3] = {tp, tu, tv};
+  const void *const src[3] = {h->tend[0], h->tend[1], h->tend[2]};
+  CCS_TRY(h, copy_field_runs(dst, src, 3, (size_t)h->L.field * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
   CCS_TRY(h, cudaStreamSynchronize(h->stream));
   return CCS_OK;
 }
@@ -1010,30 +1001,6 @@ static void mixed_handle_destroy(ccs_handle *h) {
   if (M->d_work) cudaFree(M->d_work);
   delete M;
   h->mixed = nullptr;
-}
-
-// Copies n fields of `bytes` each (dst[q] <- src[q], NULL entries skipped), one
-// cudaMemcpyAsync per run of fields whose destination and source both continue the
-// previous field's: a caller whose host arrays are consecutive slices of one
-// page-locked block gets one copy per direction, which the host link overlaps
-// with the other direction better than many smaller copies.
-static cudaError_t copy_field_runs(void *const *dst, const void *const *src, int n, size_t bytes,
-                                   cudaMemcpyKind kind, cudaStream_t s) {
-  int q = 0;
-  while (q < n) {
-    if (!dst[q] || !src[q]) {
-      q++;
-      continue;
-    }
-    int e = q + 1;
-    while (e < n && dst[e] && src[e] && (char *)dst[e] == (char *)dst[e - 1] + bytes &&
-           (const char *)src[e] == (const char *)src[e - 1] + bytes)
-      e++;
-    const cudaError_t err = cudaMemcpyAsync(dst[q], src[q], (size_t)(e - q) * bytes, kind, s);
-    if (err != cudaSuccess) return err;
-    q = e;
-  }
-  return cudaSuccess;
 }
 
 static int mixed_set_state(ccs_handle *h, const ccs_state_view *s, bool sync) {
