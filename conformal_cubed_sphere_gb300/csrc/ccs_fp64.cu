@@ -766,6 +766,9 @@ namespace {
 using F64T0 = F64Tile<32, 8, 384, 2>;
 using F64T1 = F64Tile<16, 16, 384, 2>;
 using F64T2 = F64Tile<64, 4, 384, 1>;
+// parts of 16 x 8 cells, three CTAs an SM
+using F64H0 = F64Tile<16, 8, 288, 3, 32, 8>;
+using F64H1 = F64Tile<16, 8, 288, 3, 16, 16>;
 // parts of 8 x 8 cells: nine warps hold all its face sides at once
 using F64S0 = F64Tile<8, 8, 288, 2, 32, 8>;
 using F64S1 = F64Tile<8, 8, 288, 2, 16, 16>;
@@ -823,25 +826,30 @@ int f64_max_grid(int var, int device) {
   }
 }
 
-// A launch whose items in four parts still fit the resident CTAs (grid) runs in parts: the
-// 256 cells of an item take one CTA 54 us whatever the number of items, its parts of 64
-// cells 24 us on an SM of their own and 30 us two to an SM (C24: 61 -> 24 us a stage, C48
-// 61 -> 30; C64, with 96 items, 54 us whole and 58 in parts).  64 x 4 items have no such parts.
+// The 256 cells of an item take one CTA 54 us alone on its SM, and two CTAs 84 us.  Small
+// launches therefore run their items in parts, as long as all parts are resident:
+//   in four (8 x 8 cells) when there are at most two an SM: C24 61 -> 23 us a stage, C48 61
+//   -> 29.5 (C64, with 96 items: 58, in two 49, whole 54)
+//   in two (16 x 8 cells) when there are at most three an SM: C64 54 -> 49, C96 84 -> 67
+//   (larger grids lose by the halo cells of the parts: C192 245 -> 260, C384 921 -> 985)
+// grid: the resident CTAs of whole items, two an SM.  64 x 4 items have no such parts.
 cudaError_t launch_f64_stage(int var, const F64Stage *d_stages, const WorkItem *d_work, int nwork, int grid,
                              cudaStream_t s, bool chained) {
-#ifdef CCS_BOUNDS
-  const bool split = var != 2 && nwork <= 12;  // (the checked build reaches both on small grids)
+#ifdef CCS_BOUNDS  // (the checked build reaches all three on small grids)
+  const int parts = nwork <= 12 ? 4 : nwork <= 24 ? 2 : 1;
 #else
-  const bool split = var != 2 && 4 * nwork <= grid;
+  const int parts = 4 * nwork <= grid ? 4 : 4 * nwork <= 3 * grid ? 2 : 1;
 #endif
   switch (var) {
     case 1:
-      return split ? f64_launch_parts<F64S1>(d_stages, d_work, nwork, s, chained)
-                   : f64_launch<F64T1>(d_stages, d_work, nwork, grid, s, chained);
+      if (parts == 4) return f64_launch_parts<F64S1>(d_stages, d_work, nwork, s, chained);
+      if (parts == 2) return f64_launch_parts<F64H1>(d_stages, d_work, nwork, s, chained);
+      return f64_launch<F64T1>(d_stages, d_work, nwork, grid, s, chained);
     case 2: return f64_launch<F64T2>(d_stages, d_work, nwork, grid, s, chained);
     default:
-      return split ? f64_launch_parts<F64S0>(d_stages, d_work, nwork, s, chained)
-                   : f64_launch<F64T0>(d_stages, d_work, nwork, grid, s, chained);
+      if (parts == 4) return f64_launch_parts<F64S0>(d_stages, d_work, nwork, s, chained);
+      if (parts == 2) return f64_launch_parts<F64H0>(d_stages, d_work, nwork, s, chained);
+      return f64_launch<F64T0>(d_stages, d_work, nwork, grid, s, chained);
   }
 }
 

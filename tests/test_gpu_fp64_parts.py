@@ -1,5 +1,5 @@
-"""FP64 lane: small launches run their work items in parts of 8 x 8 cells, larger ones
-whole; both sides of the line, with partial tiles and parts beyond the panel's edge,
+"""FP64 lane: small launches run their work items in parts of 8 x 8 or 16 x 8 cells, larger
+ones whole; both sides of the lines, with partial tiles and parts beyond the panel's edge,
 give the oracle's bits."""
 import pytest
 
@@ -12,8 +12,9 @@ pytestmark = pytest.mark.gpu
 
 
 # N = 4: one part of an item holds all cells; 12 and 41: parts beyond the edge; 48: the
-# largest grid in parts on two CTAs an SM; 52 and 68: whole items, the last ones partial
-@pytest.mark.parametrize("N", [4, 12, 41, 48, 52, 68])
+# largest grid in quarters; 52 and 95: halves, the last ones partial or beyond the edge;
+# 100: whole items, the last ones partial
+@pytest.mark.parametrize("N", [4, 12, 41, 48, 52, 95, 100])
 @pytest.mark.parametrize("var", [0, 1])
 def test_parts_and_whole_items_bitwise(N, var):
     ediss = L.CCS_EDISS_RECONSTRUCT if var else L.CCS_EDISS_ZERO
