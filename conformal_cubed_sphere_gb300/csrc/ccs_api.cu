@@ -1254,7 +1254,7 @@ static int set_variant(ccs_handle *h, int var) {
 }
 
 // Mean time of one stage launch with the handle's current variant, over the RK
-// stages before the last one, in step order.  Those stages read the state and
+// stages before the last one, in step order and chained as a step's stages are.  Those stages read the state and
 // write only stage scratch (the next stage's input and the RK accumulator); the
 // last stage, which writes the state, is the only one left out, so timing leaves
 // the state unchanged.
@@ -1267,9 +1267,9 @@ static int time_stages(ccs_handle *h, int reps, double *us) {
   auto launch = [&](int k) -> cudaError_t {
     if (mx) {
       MixedLane *M = h->mixed;
-      return mixed_launch(h, M->d_stages + k);
+      return mixed_launch(h, M->d_stages + k, k > 0);
     }
-    return launch_f64_stage(h->var, h->d_stages + k, h->d_work, h->nwork, h->grid, h->stream);
+    return launch_f64_stage(h->var, h->d_stages + k, h->d_work, h->nwork, h->grid, h->stream, k > 0);
   };
   cudaError_t e = launch(0);  // warm-up
   for (int r = 0; r < reps && e == cudaSuccess; r++) {
@@ -1560,7 +1560,7 @@ static int group_time_stages(ccs_batch *b, BatchGroup &g, int reps, double *us) 
   if (e == cudaSuccess) e = group_launch(g, 0, false);  // warm-up
   if (e == cudaSuccess) e = cudaEventRecord(e0, g.stream);
   for (int r = 0; r < reps && e == cudaSuccess; r++)
-    for (int k = 0; k < nst && e == cudaSuccess; k++) e = group_launch(g, k, false);
+    for (int k = 0; k < nst && e == cudaSuccess; k++) e = group_launch(g, k, false, k > 0);
   if (e == cudaSuccess) e = cudaEventRecord(e1, g.stream);
   if (e == cudaSuccess) e = cudaEventSynchronize(e1);
   float ms = 0.f;
