@@ -149,7 +149,8 @@ struct ccs_handle {
   int var = 0;  // tile variant of the FP64 stage kernel (kF64Tiles)
   int op = CCS_OP_WENO;  // spatial operator (ccs_set_operator)
   bool sphere_valid = false;
-  cudaGraphExec_t g_step = nullptr, g_step_sw = nullptr;
+  cudaGraphExec_t g_step = nullptr, g_step_sw = nullptr;  // one step, one with the sphere winds
+  cudaGraphExec_t g_steps = nullptr;                      // kGraphSteps steps
   // timing
   bool timing = false;
   cudaEvent_t ev0 = nullptr, ev1 = nullptr;
@@ -165,6 +166,12 @@ struct ccs_handle {
 };
 
 static const int kDiagBlocks = 512;
+
+// Steps of the graph that a run of many steps replays: consecutive graphs leave the GPU
+// idle for about 4 us, as long as a stage of a small grid (mixed C48 6.2 -> 5.1 us a stage,
+// C96 7.7 -> 6.7, C384 33.4 -> 32.7; FP64 C48 29.5 -> 28.6).  Captured when a call asks for
+// at least twice as many steps, so that short calls do not pay for the larger graph.
+constexpr int kGraphSteps = 8;
 
 // Copies n fields of `bytes` each (dst[q] <- src[q], NULL entries skipped), one
 // cudaMemcpyAsync per run of fields whose destination and source both continue the
@@ -405,12 +412,14 @@ static int build_f64_lane(ccs_handle *h) {
   return CCS_OK;
 }
 
-// enqueue one step; with_sw: the final stage also writes the sphere winds
-static int f64_enqueue_step(ccs_handle *h, bool with_sw) {
+// enqueue one step; with_sw: the final stage also writes the sphere winds; first: the
+// launch before it in the stream is not the previous step's last stage
+static int f64_enqueue_step(ccs_handle *h, bool with_sw, bool first = true) {
   for (int k = 0; k < h->n_rk; k++) {
     const F64Stage *d = h->d_stages + ((k == h->n_rk - 1 && with_sw) ? h->n_rk : k);
     if (h->timing) CCS_TRY(h, cudaEventRecord(h->ev0, h->stream));
-    CCS_TRY(h, launch_f64_stage(h->var, d, h->d_work, h->nwork, h->grid, h->stream, k > 0 && !h->timing));
+    CCS_TRY(h, launch_f64_stage(h->var, d, h->d_work, h->nwork, h->grid, h->stream,
+                                (k > 0 || !first) && !h->timing));
     if (h->timing) {
       CCS_TRY(h, cudaEventRecord(h->ev1, h->stream));
       CCS_TRY(h, cudaEventSynchronize(h->ev1));
@@ -423,12 +432,14 @@ static int f64_enqueue_step(ccs_handle *h, bool with_sw) {
   return CCS_OK;
 }
 
-static int f64_capture(ccs_handle *h, bool with_sw, cudaGraphExec_t *out) {
+// captures n steps, the last with with_sw, as one graph
+static int f64_capture(ccs_handle *h, int n, bool with_sw, cudaGraphExec_t *out) {
   cudaGraph_t g = nullptr;
   CCS_TRY(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
   const bool t = h->timing;
   h->timing = false;
-  int rc = f64_enqueue_step(h, with_sw);
+  int rc = CCS_OK;
+  for (int s = 0; s < n && !rc; s++) rc = f64_enqueue_step(h, with_sw && s == n - 1, s == 0);
   h->timing = t;
   cudaError_t e = cudaStreamEndCapture(h->stream, &g);
   if (rc) return rc;
@@ -454,12 +465,19 @@ static int f64_step(ccs_handle *h, int nsteps, bool sync) {
     }
   } else {
     if (!h->g_step) {
-      int rc = f64_capture(h, false, &h->g_step);
+      int rc = f64_capture(h, 1, false, &h->g_step);
       if (rc) return rc;
-      rc = f64_capture(h, true, &h->g_step_sw);
+      rc = f64_capture(h, 1, true, &h->g_step_sw);
       if (rc) return rc;
     }
-    for (int s = 0; s < nsteps - 1; s++) CCS_TRY(h, cudaGraphLaunch(h->g_step, h->stream));
+    if (nsteps > 2 * kGraphSteps && !h->g_steps) {
+      int rc = f64_capture(h, kGraphSteps, false, &h->g_steps);
+      if (rc) return rc;
+    }
+    int s = nsteps - 1;
+    if (h->g_steps)
+      for (; s >= kGraphSteps; s -= kGraphSteps) CCS_TRY(h, cudaGraphLaunch(h->g_steps, h->stream));
+    for (; s > 0; s--) CCS_TRY(h, cudaGraphLaunch(h->g_step, h->stream));
     CCS_TRY(h, cudaGraphLaunch(h->g_step_sw, h->stream));
   }
   h->sphere_valid = true;
@@ -614,6 +632,7 @@ void ccs_destroy(ccs_handle *h) {
   if (h->stream) cudaStreamSynchronize(h->stream);
   if (h->g_step) cudaGraphExecDestroy(h->g_step);
   if (h->g_step_sw) cudaGraphExecDestroy(h->g_step_sw);
+  if (h->g_steps) cudaGraphExecDestroy(h->g_steps);
   if (h->sbuf) cudaFree(h->sbuf);
   if (h->d_stages) cudaFree(h->d_stages);
   if (h->d_work) cudaFree(h->d_work);
@@ -782,7 +801,13 @@ struct MixedLane {
   int var = 0;  // tile variant of the mixed stage kernel (kMxTiles)
   double phibar = 0.;
   bool have_phibar = false;
-  cudaGraphExec_t g_step = nullptr;
+  cudaGraphExec_t g_step = nullptr;   // one step
+  cudaGraphExec_t g_steps = nullptr;  // kGraphSteps steps
+  void drop_graphs() {
+    if (g_step) cudaGraphExecDestroy(g_step);
+    if (g_steps) cudaGraphExecDestroy(g_steps);
+    g_step = g_steps = nullptr;
+  }
 };
 
 static int mixed_mesh_setup(ccs_handle *h, DeviceMesh *dm, const ccs_mesh_view *mv) {
@@ -977,10 +1002,7 @@ static int mixed_build_stages(ccs_handle *h) {
   CCS_TRY(h, cudaMemcpyAsync(M->d_stages, M->h_stages.data(), M->h_stages.size() * sizeof(MixedStage),
                              cudaMemcpyHostToDevice, h->stream));
   CCS_TRY(h, cudaStreamSynchronize(h->stream));
-  if (M->g_step) {
-    cudaGraphExecDestroy(M->g_step);
-    M->g_step = nullptr;
-  }
+  M->drop_graphs();
   return CCS_OK;
 }
 
@@ -989,7 +1011,7 @@ static void mixed_handle_destroy(ccs_handle *h) {
   if (!M) return;
   if (M->cin) cudaStreamSynchronize(M->cin);
   if (M->cout) cudaStreamSynchronize(M->cout);
-  if (M->g_step) cudaGraphExecDestroy(M->g_step);
+  M->drop_graphs();
   if (M->buf) cudaFree(M->buf);
   for (int k = 0; k < 2; k++)
     for (cudaEvent_t e : {M->in_ready[k], M->in_free[k], M->out_ready[k], M->out_free[k]})
@@ -1081,11 +1103,13 @@ static int mixed_sync(ccs_handle *h) {
   return CCS_OK;
 }
 
-static int mixed_enqueue_step(ccs_handle *h) {
+// enqueue one step; first: the launch before it in the stream is not the previous step's
+// last stage
+static int mixed_enqueue_step(ccs_handle *h, bool first = true) {
   MixedLane *M = h->mixed;
   for (int k = 0; k < M->n_rk; k++) {
     if (h->timing) CCS_TRY(h, cudaEventRecord(h->ev0, h->stream));
-    CCS_TRY(h, mixed_launch(h, M->d_stages + k, k > 0 && !h->timing));
+    CCS_TRY(h, mixed_launch(h, M->d_stages + k, (k > 0 || !first) && !h->timing));
     if (h->timing) {
       CCS_TRY(h, cudaEventRecord(h->ev1, h->stream));
       CCS_TRY(h, cudaEventSynchronize(h->ev1));
@@ -1095,6 +1119,21 @@ static int mixed_enqueue_step(ccs_handle *h) {
       h->launches++;
     }
   }
+  return CCS_OK;
+}
+
+// captures n steps as one graph
+static int mixed_capture(ccs_handle *h, int n, cudaGraphExec_t *out) {
+  cudaGraph_t g = nullptr;
+  CCS_TRY(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
+  int rc = CCS_OK;
+  for (int s = 0; s < n && !rc; s++) rc = mixed_enqueue_step(h, s == 0);
+  cudaError_t e = cudaStreamEndCapture(h->stream, &g);
+  if (rc) return rc;
+  CCS_TRY(h, e);
+  e = cudaGraphInstantiate(out, g, 0);
+  cudaGraphDestroy(g);
+  CCS_TRY(h, e);
   return CCS_OK;
 }
 
@@ -1108,18 +1147,18 @@ static int mixed_step(ccs_handle *h, int nsteps, bool sync) {
       if (rc) return rc;
     }
   } else {
-    if (!M->g_step) {
-      cudaGraph_t g = nullptr;
-      CCS_TRY(h, cudaStreamBeginCapture(h->stream, cudaStreamCaptureModeThreadLocal));
-      int rc = mixed_enqueue_step(h);
-      cudaError_t e = cudaStreamEndCapture(h->stream, &g);
+    if (nsteps >= 2 * kGraphSteps && !M->g_steps) {
+      int rc = mixed_capture(h, kGraphSteps, &M->g_steps);
       if (rc) return rc;
-      CCS_TRY(h, e);
-      e = cudaGraphInstantiate(&M->g_step, g, 0);
-      cudaGraphDestroy(g);
-      CCS_TRY(h, e);
     }
-    for (int s = 0; s < nsteps; s++) CCS_TRY(h, cudaGraphLaunch(M->g_step, h->stream));
+    if (!M->g_step) {
+      int rc = mixed_capture(h, 1, &M->g_step);
+      if (rc) return rc;
+    }
+    int s = nsteps;
+    if (M->g_steps)
+      for (; s >= kGraphSteps; s -= kGraphSteps) CCS_TRY(h, cudaGraphLaunch(M->g_steps, h->stream));
+    for (; s > 0; s--) CCS_TRY(h, cudaGraphLaunch(M->g_step, h->stream));
   }
   if (sync) CCS_TRY(h, cudaStreamSynchronize(h->stream));
   return CCS_OK;
@@ -1236,10 +1275,7 @@ static int set_variant(ccs_handle *h, int var) {
     if (rc) return rc;
     M->var = var;
     M->grid = mixed_max_grid(var, dev);
-    if (M->g_step) {
-      cudaGraphExecDestroy(M->g_step);
-      M->g_step = nullptr;
-    }
+    M->drop_graphs();
   } else {
     if (var == h->var && h->d_work) return CCS_OK;
     int rc = build_work(h, kF64Tiles[var], &h->d_work, &h->nwork);
@@ -1248,7 +1284,8 @@ static int set_variant(ccs_handle *h, int var) {
     h->grid = f64_max_grid(var, dev);
     if (h->g_step) cudaGraphExecDestroy(h->g_step);
     if (h->g_step_sw) cudaGraphExecDestroy(h->g_step_sw);
-    h->g_step = h->g_step_sw = nullptr;
+    if (h->g_steps) cudaGraphExecDestroy(h->g_steps);
+    h->g_step = h->g_step_sw = h->g_steps = nullptr;
   }
   return CCS_OK;
 }
@@ -1364,7 +1401,8 @@ struct ccs_batch {
   cudaEvent_t fork = nullptr;
   cudaEvent_t after = nullptr;  // end of the last enqueued step, for the members' streams
   int device = 0;
-  cudaGraphExec_t g_step = nullptr, g_step_sw = nullptr;
+  cudaGraphExec_t g_step = nullptr, g_step_sw = nullptr;  // one step, one with the FP64 members' sphere winds
+  cudaGraphExec_t g_steps = nullptr;                      // kGraphSteps steps
   std::string err;
 };
 
@@ -1418,14 +1456,15 @@ static int group_set_var(ccs_batch *b, BatchGroup &g, int var) {
   return CCS_OK;
 }
 
-// One step of every group: the groups fork from the batch stream, run their RK
-// stages on their own streams (an FP64 group is FP64-issue bound and a mixed group
+// n steps of every group (with_sw: the last one with the sphere winds): the groups fork
+// from the batch stream, run their RK stages on their own streams (an FP64 group is FP64-issue bound and a mixed group
 // FP32 / latency bound, so they share the SMs well) and join back.
-static int batch_enqueue(ccs_batch *b, bool with_sw) {
+static int batch_enqueue(ccs_batch *b, int n, bool with_sw) {
   BATCH_TRY(b, cudaEventRecord(b->fork, b->stream));
   for (auto &g : b->groups) {
     BATCH_TRY(b, cudaStreamWaitEvent(g.stream, b->fork, 0));
-    for (int k = 0; k < g.n_rk; k++) BATCH_TRY(b, group_launch(g, k, with_sw, k > 0));
+    for (int s = 0; s < n; s++)
+      for (int k = 0; k < g.n_rk; k++) BATCH_TRY(b, group_launch(g, k, with_sw && s == n - 1, s > 0 || k > 0));
     BATCH_TRY(b, cudaEventRecord(g.done, g.stream));
     BATCH_TRY(b, cudaStreamWaitEvent(b->stream, g.done, 0));
   }
@@ -1596,7 +1635,8 @@ extern "C" int ccs_batch_autotune(ccs_batch *b, int reps) {
   }
   if (b->g_step) cudaGraphExecDestroy(b->g_step);
   if (b->g_step_sw) cudaGraphExecDestroy(b->g_step_sw);
-  b->g_step = b->g_step_sw = nullptr;
+  if (b->g_steps) cudaGraphExecDestroy(b->g_steps);
+  b->g_step = b->g_step_sw = b->g_steps = nullptr;
   return CCS_OK;
 }
 
@@ -1613,10 +1653,10 @@ extern "C" int ccs_batch_info(ccs_batch *b, int *launches_per_stage, int max_gro
   return CCS_OK;
 }
 
-static int batch_capture(ccs_batch *b, bool with_sw, cudaGraphExec_t *out) {
+static int batch_capture(ccs_batch *b, int n, bool with_sw, cudaGraphExec_t *out) {
   cudaGraph_t g = nullptr;
   BATCH_TRY(b, cudaStreamBeginCapture(b->stream, cudaStreamCaptureModeThreadLocal));
-  int rc = batch_enqueue(b, with_sw);
+  int rc = batch_enqueue(b, n, with_sw);
   cudaError_t e = cudaStreamEndCapture(b->stream, &g);
   if (rc) {
     if (g) cudaGraphDestroy(g);
@@ -1635,8 +1675,12 @@ static int batch_step(ccs_batch *b, int nsteps, bool sync) {
   if (nsteps == 0) return CCS_OK;
   BATCH_TRY(b, cudaSetDevice(b->device));
   if (!b->g_step) {
-    int rc = batch_capture(b, false, &b->g_step);
-    if (!rc) rc = batch_capture(b, true, &b->g_step_sw);
+    int rc = batch_capture(b, 1, false, &b->g_step);
+    if (!rc) rc = batch_capture(b, 1, true, &b->g_step_sw);
+    if (rc) return rc;
+  }
+  if (nsteps > 2 * kGraphSteps && !b->g_steps) {
+    int rc = batch_capture(b, kGraphSteps, false, &b->g_steps);
     if (rc) return rc;
   }
   // the step starts after the members' own pending work (an asynchronous upload and
@@ -1646,7 +1690,10 @@ static int batch_step(ccs_batch *b, int nsteps, bool sync) {
     BATCH_TRY(b, cudaEventRecord(h->ev_order, h->stream));
     BATCH_TRY(b, cudaStreamWaitEvent(b->stream, h->ev_order, 0));
   }
-  for (int s = 0; s < nsteps - 1; s++) BATCH_TRY(b, cudaGraphLaunch(b->g_step, b->stream));
+  int s = nsteps - 1;
+  if (b->g_steps)
+    for (; s >= kGraphSteps; s -= kGraphSteps) BATCH_TRY(b, cudaGraphLaunch(b->g_steps, b->stream));
+  for (; s > 0; s--) BATCH_TRY(b, cudaGraphLaunch(b->g_step, b->stream));
   BATCH_TRY(b, cudaGraphLaunch(b->g_step_sw, b->stream));
   BATCH_TRY(b, cudaEventRecord(b->after, b->stream));
   for (ccs_handle *h : b->members) BATCH_TRY(b, cudaStreamWaitEvent(h->stream, b->after, 0));
@@ -1666,6 +1713,7 @@ extern "C" void ccs_batch_destroy(ccs_batch *b) {
   if (b->stream) cudaStreamSynchronize(b->stream);
   if (b->g_step) cudaGraphExecDestroy(b->g_step);
   if (b->g_step_sw) cudaGraphExecDestroy(b->g_step_sw);
+  if (b->g_steps) cudaGraphExecDestroy(b->g_steps);
   for (auto &g : b->groups) {
     if (g.d_stages) cudaFree(g.d_stages);
     if (g.d_work) cudaFree(g.d_work);
