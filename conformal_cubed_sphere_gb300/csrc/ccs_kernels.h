@@ -51,8 +51,8 @@ cudaError_t launch_stage(void (*kernel)(P...), int grid, int block, int smem, cu
 // have room: mixed C150 10.3 -> 12.0 us a stage)
 __device__ __forceinline__ void stage_release() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // waits until the previous stage of a chained launch has ended and its writes are visible
-// (returns at once in other launches).  Whatever a stage writes is read after this and
-// through L2 (__ldcg): this SM's L1 may hold lines that the previous stage read.
+// (returns at once in other launches).  Whatever a stage writes is read after this, and
+// never as read-only data (__ldg): it changes while the kernel is already running.
 __device__ __forceinline__ void stage_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 #endif
 
