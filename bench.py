@@ -124,7 +124,7 @@ def _peaks():
 
 
 # the sources of the stage kernels whose ncu counters profiles/roofline_traffic.json holds
-KERNEL_SOURCES = ("ccs_mixed.cu", "ccs_fp64.cu", "ccs_kernels.h", "ccs_internal.h")
+KERNEL_SOURCES = ("ccs_mixed.cu", "ccs_fp64.cu", "ccs_softfp.cuh", "ccs_kernels.h", "ccs_internal.h")
 
 
 def kernel_sources_hash() -> str:
@@ -431,7 +431,7 @@ def run_ensemble(torch, members_per_gpu: int, steps: int, warmup: int) -> dict:
         "hbm_frac": alg / hbm, "alg_GBs": alg, "launches_per_stage": launches,
         "tile_variant": groups[0][1] if groups else None,
         "variant": variant_name("mixed", groups[0][1]) if groups else None,
-        "how": "one graph per step, one persistent launch per RK stage over all members' tiles, CUDA events on "
+        "how": "step graphs, one persistent launch per RK stage over all members' tiles, CUDA events on "
                "the batch stream; sequential = each member's own handle (graph per step) one after another, "
                "host-timed; inputs larger than L2",
     }
@@ -492,8 +492,8 @@ def run_uneven(torch, steps: int, warmup: int) -> dict:
         "launches_per_stage": launches, "tile_variants": tiles, "variants": names, "fp64_cells": cells64,
         "mixed_cells": cells32,
         "instances": len(members),
-        "how": "29 instances with per-instance CFL dt, one FP64 member per resolution below C384; one graph per "
-               "step, each lane's stages on its own stream; CUDA events on the batch stream",
+        "how": "29 instances with per-instance CFL dt, one FP64 member per resolution below C384; step graphs, "
+               "each lane's stages on its own stream; CUDA events on the batch stream",
         "mixed_members_alone": {
             "cell_steps_per_s": ws * cells32 * steps / t32, "ms_per_step": 1e3 * t32 / steps,
             "hbm_frac": alg32 / _peaks()[0], "alg_GBs": ws * alg32, "launches_per_stage": n32,

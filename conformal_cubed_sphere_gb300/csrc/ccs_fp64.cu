@@ -11,8 +11,8 @@
 // weights and the constant multiples of cell values run on the integer pipes
 // (ccs_softfp.cuh), which also round like IEEE; what stays is written as FMAs (F64Ops).
 // C384 stage with 16 x 16 tiles: 3160 us with every operation on the FP64 pipe, 1219 with
-// shared products and integer quotients, 946 now; FP64 thread instructions per cell and
-// stage 1780 -> 490.  Products of two variables (squares, weight times stencil) are no
+// shared products and integer quotients, 921 now; FP64 thread instructions per cell and
+// stage 1780 -> 485.  Products of two variables (squares, weight times stencil) are no
 // faster in integers (+2 %) and stay.
 //
 // A CTA owns a tile of F64_TX x F64_TY interior cells of one panel.  It stages the

@@ -117,7 +117,7 @@ struct MixedStage {
 struct TileShape {
   int tx, ty;
 };
-constexpr int F64_NVAR = 3;  // 32 x 8, 16 x 16, 64 x 4 (256 threads, one cell each in phase 3)
+constexpr int F64_NVAR = 3;  // 32 x 8, 16 x 16, 64 x 4 (384 threads; small launches run 8 x 8 or 16 x 8 parts)
 constexpr TileShape kF64Tiles[F64_NVAR] = {{32, 8}, {16, 16}, {64, 4}};
 // Mixed lane: tile shape x halo-staging schedule of phase 1.  kStageLoads: each
 // thread loads its cells' raw inputs into registers and stores the derived cell

@@ -994,6 +994,8 @@ int mixed_max_grid(int var, int device) {
 //   16 x 16, four faces a segment, while all of them are resident, six an SM (about C190):
 //   C112 11.8 -> 9.6, C128 11.8 -> 9.7, C160 11.8 -> 10.8, C192 14.0 -> 13.3 (C208 15.4 ->
 //   17.9: the shorter segments compute a quarter more cells, and a second wave begins)
+// (both sides in unchained launches; chained, eight steps a graph and with the 16 x 8 tiles'
+// operands in flight before the wait: C24 4.6, C48 5.1, C96 6.7, C128 9.3, C192 12.8)
 // Same bits in every tile shape.
 cudaError_t launch_mixed_stage(int var, bool central, bool ediss, const MixedStage *d_stages,
                                const WorkItem *d_work, int nwork, int grid, cudaStream_t s,

@@ -179,7 +179,8 @@ int ccs_set_operator(ccs_handle *h, int op);
  * cells' raw inputs into registers and stores the derived quantities), 2: 32x32
  * and 3: 32x16 with asynchronous copies (the raw inputs of all of a thread's cells
  * go into shared memory at once, then are derived in place).  Every variant
- * computes the same per-cell arithmetic, so results do not depend on the choice.  ccs_autotune times the handle's RK stages before the last one (they write
+ * computes the same per-cell arithmetic, so results do not depend on the choice; a
+ * launch with few work items runs smaller parts of them, whatever the variant.  ccs_autotune times the handle's RK stages before the last one (they write
  * only stage scratch, so the state is unchanged), `reps` rounds with each variant
  * after one warm-up launch, and keeps the fastest mean stage time; the choice is cached per (device, lane, N,
  * halo) for the process, and later calls with force = 0 reuse it without timing.
