@@ -338,6 +338,14 @@ static int build_work(ccs_handle *h, TileShape ts, WorkItem **d_work, int *nwork
   return CCS_OK;
 }
 
+// the grid's divisor b > 0 for the integer quotients; y = 0, IEEE division, outside
+// [2^-400, 2^300), where a quotient might leave the normal range
+static softfp::Divisor grid_divisor(double b) {
+  softfp::Divisor d = softfp::divisor(softfp::unpack(b));
+  if (!(b >= 0x1p-400 && b < 0x1p300)) d.y = 0u;
+  return d;
+}
+
 static int build_f64_lane(ccs_handle *h) {
   const Layout &L = h->L;
   const size_t nf = (size_t)L.field;
@@ -366,10 +374,10 @@ static int build_f64_lane(ccs_handle *h) {
   base.accphiG = h->acc[0]; base.accu = h->acc[1]; base.accv = h->acc[2];
   base.dx = c.dx; base.dy = c.dy;
   base.dx60 = 60. * c.dx; base.dy60 = 60. * c.dy;
-  base.by_dx = softfp::divisor(softfp::unpack(base.dx));
-  base.by_dy = softfp::divisor(softfp::unpack(base.dy));
-  base.by_dx60 = softfp::divisor(softfp::unpack(base.dx60));
-  base.by_dy60 = softfp::divisor(softfp::unpack(base.dy60));
+  base.by_dx = grid_divisor(base.dx);
+  base.by_dy = grid_divisor(base.dy);
+  base.by_dx60 = grid_divisor(base.dx60);
+  base.by_dy60 = grid_divisor(base.dy60);
   base.ediss = c.e_dissipation;
   base.op = h->op;
   auto mk = [&](int kind, int in, int out, double c1) {

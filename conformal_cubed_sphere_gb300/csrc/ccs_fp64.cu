@@ -186,19 +186,20 @@ struct F64Ops {
   }
 };
 
-// phiG / sqrtG from the grid's reciprocals y = RN(1 / sqrtG); a phiG so small that the
-// quotient might not be normal takes IEEE division
+// phiG / sqrtG from the grid's reciprocals y = RN(1 / sqrtG), which are zero where sqrtG is
+// not in [2^-400, 2^300); there, and for a phiG whose quotient might not be normal, IEEE
+// division
 __device__ __forceinline__ double div_depth(const F64Ops &f, double x, double b, double y) {
   const unsigned e = ((unsigned)__double2hiint(x) >> 20) & 0x7ffu;
-  if (e < 257u && x != 0.) return x / b;
+  if ((e - 400u >= 1200u && x != 0.) || __double2hiint(y) == 0) return x / b;
   return f.div_const(x, b, y);
 }
 
-// x / b on the integer pipes, b prepared by the host; values whose quotient might leave
-// the normal range (and zeros) take IEEE division
+// x / b on the integer pipes, b prepared by the host (y zero: b not in [2^-400, 2^300));
+// values whose quotient might leave the normal range (and zeros) take IEEE division
 __device__ __forceinline__ double div_by(double x, const softfp::Divisor &d, double b) {
   const uint32_t h = (uint32_t)__double2hiint(x);
-  if (((h >> 20) & 0x7ffu) - 400u >= 1200u) return x / b;
+  if (((h >> 20) & 0x7ffu) - 400u >= 1200u || d.y == 0u) return x / b;
   const double q = softfp::round_double(softfp::div(softfp::unpack(x), d));
   return __hiloint2double((int)((uint32_t)__double2hiint(q) | (h & 0x80000000u)), __double2loint(q));
 }
@@ -862,7 +863,9 @@ __global__ void mesh_products_kernel(Layout L, MeshF64 m, double *__restrict__ o
     const int ia = (int)(q % L.nh), ja = (int)((q / L.nh) % L.nh), p = (int)(q / ((int64_t)L.nh * L.nh));
     const int64_t c = ia + (int64_t)L.pitch * ja + L.panel * p;
     out[c] = m.sqrtG[c] * m.f[c];
-    out[L.field + c] = 1. / m.sqrtG[c];
+    // (for div_depth)
+    const unsigned e = ((unsigned)__double2hiint(m.sqrtG[c]) >> 20) & 0x7ffu;
+    out[L.field + c] = e - 623u < 700u ? 1. / m.sqrtG[c] : 0.;
     if (ia + 1 < L.nh) out[2 * L.field + c] = 0.5 * (m.ig11[c + 1] + m.ig11[c]);
     if (ja + 1 < L.nh) out[3 * L.field + c] = 0.5 * (m.ig22[c + L.pitch] + m.ig22[c]);
   }

@@ -1,6 +1,8 @@
 """FP64 lane: tiles whose field values leave the exponent window of the integer
 arithmetic take the FP64 instructions, the others the integer ones; both, and the
 mixture, give the oracle's bits."""
+import copy
+
 import numpy as np
 import pytest
 
@@ -47,3 +49,13 @@ def test_constant_state():
     s["phi"][:] = 8.0e4
     s["phiG"] = s["phi"] * mesh.sqrtG
     _check(mesh, s, dt, L.CCS_EDISS_ZERO, 3)
+
+
+@pytest.mark.parametrize("k", [-500, -405, -390, 280, 310, 480])
+def test_grid_spacings_beyond_the_quotients_range(k):
+    """dx and dy scaled by 2^k, dt with small ones: the integer quotients by dx, dy, 60 dx and
+    60 dy end at 2^-400 and 2^300."""
+    mesh, s, dt = seeded_case(16, 3, seed=7, oro=True)
+    mesh = copy.copy(mesh)
+    mesh.dx, mesh.dy = mesh.dx * 2.0 ** k, mesh.dy * 2.0 ** k
+    _check(mesh, s, dt * 2.0 ** min(k, 0), L.CCS_EDISS_RECONSTRUCT, 1)
