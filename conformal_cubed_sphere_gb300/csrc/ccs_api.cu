@@ -177,7 +177,10 @@ constexpr int kGraphSteps = 8;
 // cudaMemcpyAsync per run of fields whose destination and source both continue the
 // previous field's: a caller whose host arrays are consecutive slices of one
 // page-locked block gets one copy per direction, which the host link overlaps
-// with the other direction better than many smaller copies.
+// with the other direction better than many smaller copies.  Host arrays that abut may
+// also belong to different allocations, page-locked one by one or only some of them; CUDA
+// refuses a copy across such a border as a whole, and the run's fields are then copied
+// one by one.
 static cudaError_t copy_field_runs(void *const *dst, const void *const *src, int n, size_t bytes,
                                    cudaMemcpyKind kind, cudaStream_t s) {
   int q = 0;
@@ -190,7 +193,12 @@ static cudaError_t copy_field_runs(void *const *dst, const void *const *src, int
     while (e < n && dst[e] && src[e] && (char *)dst[e] == (char *)dst[e - 1] + bytes &&
            (const char *)src[e] == (const char *)src[e - 1] + bytes)
       e++;
-    const cudaError_t err = cudaMemcpyAsync(dst[q], src[q], (size_t)(e - q) * bytes, kind, s);
+    cudaError_t err = cudaMemcpyAsync(dst[q], src[q], (size_t)(e - q) * bytes, kind, s);
+    if (err == cudaErrorInvalidValue && e - q > 1) {
+      (void)cudaGetLastError();  // dealt with here: the next launch must not report it
+      err = cudaSuccess;
+      for (int f = q; f < e && err == cudaSuccess; f++) err = cudaMemcpyAsync(dst[f], src[f], bytes, kind, s);
+    }
     if (err != cudaSuccess) return err;
     q = e;
   }
