@@ -92,10 +92,13 @@ __global__ void courant_kernel(Layout L, const float *__restrict__ hp32, const f
   if ((threadIdx.x & 31) == 0) atomicMax(lmax, (unsigned long long)__double_as_longlong(best));
 }
 
+// A failed call is reported once, here: it is taken off the thread's last error, which
+// the next kernel launch, of this or another handle, would report as its own.
 #define CCS_TRY(h, call)                                                       \
   do {                                                                         \
     cudaError_t e_ = (call);                                                   \
     if (e_ != cudaSuccess) {                                                   \
+      (void)cudaGetLastError();                                                \
       if (h) (h)->err = std::string(#call) + ": " + cudaGetErrorString(e_);    \
       return CCS_ERR_CUDA;                                                     \
     }                                                                          \
@@ -1426,6 +1429,7 @@ struct ccs_batch {
   do {                                                                         \
     cudaError_t e_ = (call);                                                   \
     if (e_ != cudaSuccess) {                                                   \
+      (void)cudaGetLastError();                                                \
       (b)->err = std::string(#call) + ": " + cudaGetErrorString(e_);           \
       return CCS_ERR_CUDA;                                                     \
     }                                                                          \

@@ -872,8 +872,7 @@ __global__ void mesh_products_kernel(Layout L, MeshF64 m, double *__restrict__ o
 }
 
 cudaError_t launch_f64_mesh_products(const Layout &L, const MeshF64 &m, double *out, cudaStream_t s) {
-  mesh_products_kernel<<<1024, 256, 0, s>>>(L, m, out);
-  return cudaGetLastError();
+  return launch_stage(mesh_products_kernel, 1024, 256, 0, s, false, L, m, out);
 }
 
 // ---- diagnostics: calc_total_mass / calc_total_energy (diag_mod.F90:10-53) ------

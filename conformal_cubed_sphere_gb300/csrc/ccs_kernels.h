@@ -29,6 +29,8 @@ inline cudaError_t smem_attr_once(const void *fn, int smem, std::atomic<uint64_t
 // Launches a stage kernel.  chained: the launch before it in the stream is the same
 // step's previous stage, whose end the kernel itself waits for (stage_wait): its CTAs may
 // start, and read their work items and descriptors, while that stage drains.
+// Returns this launch's own status (cudaGetLastError would also report an earlier error
+// that nobody has collected).
 template <class... P, class... A>
 cudaError_t launch_stage(void (*kernel)(P...), int grid, int block, int smem, cudaStream_t s, bool chained,
                          A... args) {

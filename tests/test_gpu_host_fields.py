@@ -79,3 +79,32 @@ def test_abutting_fields_page_locked_one_by_one(precision, locked):
         g.close()
     finally:
         F.release()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+def test_a_refused_transfer_leaves_no_error_behind(precision):
+    """A field of which only a part is page-locked is refused by CUDA; the handle, and
+    handles made after it, work on."""
+    mesh, s, dt = seeded_case(58, 3, seed=4)
+    kw = dict(phi_mean=8000.0 * mesh.gravity)
+    F = Fields(1, mesh.ncell, ())
+    rt = F.torch.cuda.cudart()
+    assert int(rt.cudaHostRegister(F.a.ctypes.data, ALIGN, 0)) == 0  # the first third
+    try:
+        bad = M.State(dict(s.copy().arrays, u=F.a[0]))
+        F.a[0][:] = s["u"]
+        g = M.Stepper(mesh, dt, precision=precision, **kw)
+        g.set_state(s)
+        for again in ("fp64", "mixed"):
+            with pytest.raises(L.CCSError):
+                g.set_state(bad)
+            h = M.Stepper(mesh, dt, precision=again, **kw)
+            h.set_state(s)
+            h.step(1)
+            with pytest.raises(L.CCSError):
+                g.get_state(bad)
+            g.set_state(s)
+            g.step(1)
+            assert g.check_state() == 0 and h.check_state() == 0
+    finally:
+        rt.cudaHostUnregister(F.a.ctypes.data)
