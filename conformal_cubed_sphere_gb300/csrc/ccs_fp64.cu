@@ -602,7 +602,10 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
                             ? softfp::square_root(softfp::unpack(c2))
                             : sqrt(c2);
       double mx = f.add(fabs(uBdy), cs);
-      if (slow) {  // (a cell that is not finite keeps the reference's comparison)
+      // a wave speed that is not finite (mx >= 0, or a NaN of either sign), and a cell that is
+      // not, keep the reference's comparison and its E term
+      const bool exact = slow || (uint32_t)__double2hiint(mx) >= 0x7ff00000u;
+      if (exact) {
         const double e1 = uBdy - cs, e2 = uBdy + cs;
         mx = abs_bits(e2) > abs_bits(e1) ? fabs(e2) : fabs(e1);
       }
@@ -610,7 +613,7 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
       double ES = S.rec[1][face];
       // the never-written u_ext / v_ext slots (CCS_EDISS_ZERO) contribute mx (0 - 0): zero
       // but for a wave speed that is not finite
-      if (ediss || slow) ES = f.sub(ES, f.mul(mx, ediss ? S.rec[3][face] : 0.));
+      if (ediss || exact) ES = f.sub(ES, f.mul(mx, ediss ? S.rec[3][face] : 0.));
       S.rec[0][face] = half_of(f.sub(FS, f.mul(mx, PD)));
       S.rec[1][face] = half_of(ES);
     }

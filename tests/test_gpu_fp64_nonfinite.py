@@ -1,0 +1,43 @@
+"""FP64 lane: what is not finite comes out where the oracle has it, and every other cell
+with the oracle's bits."""
+import copy
+
+import numpy as np
+import pytest
+
+from conformal_cubed_sphere_gb300 import _lib as L
+from conformal_cubed_sphere_gb300 import model as M
+from oracle import oracle as O
+from tests.helpers import seeded_case
+
+pytestmark = pytest.mark.gpu
+
+
+def _same(a, b, m, what):
+    a, b = a[m], b[m]
+    nan = np.isnan(b)
+    assert np.array_equal(np.isnan(a), nan), (what, int(np.isnan(a).sum()), int(nan.sum()))
+    assert np.array_equal(a[~nan].view(np.int64), b[~nan].view(np.int64)), what
+    return int((~np.isfinite(b)).sum())
+
+
+# one cell's wave-speed metric negative (its square root is NaN), NaN, infinite, and so
+# large that its product with the depth overflows: the reference's never-written E slots
+# (CCS_EDISS_ZERO) then contribute inf * 0
+@pytest.mark.parametrize("value", [-1.0, np.nan, np.inf, 1.0e306])
+@pytest.mark.parametrize("ediss", [L.CCS_EDISS_ZERO, L.CCS_EDISS_RECONSTRUCT])
+@pytest.mark.parametrize("entry", [0, 3])
+def test_wave_speed_that_is_not_finite(value, ediss, entry):
+    mesh, s, dt = seeded_case(20, 3, seed=6, oro=True)
+    mesh = copy.copy(mesh)
+    mesh.matrixIG = mesh.matrixIG.copy()
+    nh = 26
+    c = (2 * nh + 12) * nh + 9  # panel 3, an interior cell
+    mesh.matrixIG.reshape(-1, 4)[c, entry] = value
+    g = M.Stepper(mesh, dt, precision="fp64", e_dissipation=ediss)
+    g.set_state(s)
+    o = O.Oracle.from_mesh(mesh, e_dissipation=ediss)
+    o.set_state(s.arrays)
+    im = mesh.interior_mask()
+    bad = [_same(a, b, im, q) for q, (a, b) in enumerate(zip(g.spatial_operator(), o.spatial_operator()))]
+    assert bad[0] > 0 and max(bad[1:]) > 0  # (phiG, and the wind across the face)
