@@ -96,34 +96,21 @@ __device__ __forceinline__ long long abs_bits(double x) {
   return __double_as_longlong(x) & 0x7fffffffffffffffLL;
 }
 
-// WENO_limiter, spatial_operators_mod.F90:282-361.
-template <int DIR>
-__device__ __forceinline__ double weno5z(double q0, double q1, double q2, double q3, double q4) {
-  // q0..q4 = Q(1..5) = field(i-2 .. i+2)
-  const double Qim2 = q0, Qim1 = q1, Qi = q2, Qip1 = q3, Qip2 = q4;
-  double s0, s1, s2, a0, a1, a2, b0, b1, b2;
+// WENO_limiter, spatial_operators_mod.F90:282-361: the "+" side.  The "-" side's formulas
+// are these with the cells in mirrored order, operation for operation, so a caller passes
+// them mirrored: the two sides of a face sit in neighbouring lanes, and with a routine each
+// a warp runs both (a C384 tendency with every tile out of the window: 6.8 -> 3.7 ms).
+__device__ __forceinline__ double weno5z(double Qim2, double Qim1, double Qi, double Qip1, double Qip2) {
   const double y3 = 1. / 3., y6 = 1. / 6., y12 = 1. / 12.;
-  if (DIR > 0) {
-    s0 = ccs_div_const(Qim2, 3., y3) - 7. / 6. * Qim1 + 11. / 6. * Qi;
-    s1 = ccs_div_const(-Qim1, 6., y6) + 5. / 6. * Qi + 1. / 3. * Qip1;
-    s2 = ccs_div_const(Qi, 3., y3) + 5. / 6. * Qip1 - 1. / 6. * Qip2;
-    a0 = Qim2 - 2. * Qim1 + Qi;
-    a1 = Qim1 - 2. * Qi + Qip1;
-    a2 = Qi - 2. * Qip1 + Qip2;
-    b0 = Qim2 - 4. * Qim1 + 3. * Qi;
-    b1 = Qim1 - Qip1;
-    b2 = 3. * Qi - 4. * Qip1 + Qip2;
-  } else {
-    s0 = ccs_div_const(Qip2, 3., y3) - 7. / 6. * Qip1 + 11. / 6. * Qi;
-    s1 = ccs_div_const(-Qip1, 6., y6) + 5. / 6. * Qi + 1. / 3. * Qim1;
-    s2 = ccs_div_const(Qi, 3., y3) + 5. / 6. * Qim1 - 1. / 6. * Qim2;
-    a0 = Qip2 - 2. * Qip1 + Qi;
-    a1 = Qip1 - 2. * Qi + Qim1;
-    a2 = Qi - 2. * Qim1 + Qim2;
-    b0 = Qip2 - 4. * Qip1 + 3. * Qi;
-    b1 = Qip1 - Qim1;
-    b2 = 3. * Qi - 4. * Qim1 + Qim2;
-  }
+  const double s0 = ccs_div_const(Qim2, 3., y3) - 7. / 6. * Qim1 + 11. / 6. * Qi;
+  const double s1 = ccs_div_const(-Qim1, 6., y6) + 5. / 6. * Qi + 1. / 3. * Qip1;
+  const double s2 = ccs_div_const(Qi, 3., y3) + 5. / 6. * Qip1 - 1. / 6. * Qip2;
+  const double a0 = Qim2 - 2. * Qim1 + Qi;
+  const double a1 = Qim1 - 2. * Qi + Qip1;
+  const double a2 = Qi - 2. * Qip1 + Qip2;
+  const double b0 = Qim2 - 4. * Qim1 + 3. * Qi;
+  const double b1 = Qim1 - Qip1;
+  const double b2 = 3. * Qi - 4. * Qip1 + Qip2;
   const double be0 = ccs_div_const(a0 * a0 * 13., 12., y12) + b0 * b0 * 0.25;
   const double be1 = ccs_div_const(a1 * a1 * 13., 12., y12) + b1 * b1 * 0.25;
   const double be2 = ccs_div_const(a2 * a2 * 13., 12., y12) + b2 * b2 * 0.25;
@@ -451,8 +438,7 @@ __device__ __forceinline__ void reconstruct(Smem<T> &S, const F64Ops &f, const d
         z += cell;
         if (minus) { st = -st; ls = -ls; }
         if (slow)
-          val = minus ? weno5z<-1>(z[2 * st], z[st], z[0], z[-st], z[-2 * st])
-                      : weno5z<1>(z[-2 * st], z[-st], z[0], z[st], z[2 * st]);
+          val = weno5z(z[-2 * st], z[-st], z[0], z[st], z[2 * st]);
         else
           val = side(f, z, st, G, face < NFX ? SGX : SGY, SAME ? st : ls, A + lcell, ls);
       }
