@@ -512,7 +512,10 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
     const Layout L = st.L;
     const int N = L.N, p = wi.panel;
     const int i0 = 1 + wi.tx * T::PX + w % T::SX * TX, j0 = 1 + wi.ty * T::PY + w / T::SX % T::SY * TY;
-    if (i0 > N || j0 > N) continue;  // (a part beyond the panel's edge)
+    if (i0 > N || j0 > N) {  // a part beyond the panel's edge
+      __syncthreads();  // (every thread has read S.st before the next part's is written)
+      continue;
+    }
     const bool ediss = st.ediss != 0;
     const int op = st.op;  // uniform over the work item
     const F64Ops f{st.one, st.neg0};
