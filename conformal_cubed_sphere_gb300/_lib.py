@@ -96,6 +96,8 @@ SIGNATURES = {
     "ccs_autotune": (C.c_int, [_vp, C.c_int, C.c_int, C.POINTER(C.c_int), _dp]),
     "ccs_set_variant": (C.c_int, [_vp, C.c_int]),
     "ccs_get_variant": (C.c_int, [_vp, C.POINTER(C.c_int), C.POINTER(C.c_int), C.POINTER(C.c_int)]),
+    "ccs_stage_tile": (C.c_int, [_vp] + [C.POINTER(C.c_int)] * 3),
+    "ccs_batch_stage_tile": (C.c_int, [_vp, C.c_int] + [C.POINTER(C.c_int)] * 3),
     "ccs_diag": (C.c_int, [_vp, _dp, _dp]),
     "ccs_diag_noalloc": (C.c_int, [C.c_int, C.c_int] + [C.c_void_p] * 9 + [_vp]),
     "ccs_batch_create": (C.c_int, [C.POINTER(_vp), C.c_int, C.POINTER(_vp)]),

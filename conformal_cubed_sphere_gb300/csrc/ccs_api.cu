@@ -1360,6 +1360,20 @@ extern "C" int ccs_get_variant(ccs_handle *h, int *var, int *tile_x, int *tile_y
   return CCS_OK;
 }
 
+extern "C" int ccs_stage_tile(ccs_handle *h, int *tile_x, int *tile_y, int *ctas) {
+  if (!h) return CCS_ERR_ARG;
+  cudaSetDevice(h->cfg.device);
+  StageTile t{};
+  if (h->cfg.precision == CCS_MIXED)
+    CCS_TRY(h, mixed_stage_tile(h->mixed->var, h->mixed->nwork, &t));
+  else
+    t = f64_stage_tile(h->var, h->nwork, h->grid);
+  if (tile_x) *tile_x = t.tx;
+  if (tile_y) *tile_y = t.ty;
+  if (ctas) *ctas = t.ctas;
+  return CCS_OK;
+}
+
 extern "C" int ccs_autotune(ccs_handle *h, int reps, int force, int *chosen, double *times_us) {
   NvtxRange nvtx("ccs_autotune");
   if (!h || reps < 1) return CCS_ERR_ARG;
@@ -1670,6 +1684,21 @@ extern "C" int ccs_batch_info(ccs_batch *b, int *launches_per_stage, int max_gro
     if (variant) variant[q] = g.var;
     if (members) members[q] = g.nmem;
   }
+  return CCS_OK;
+}
+
+extern "C" int ccs_batch_stage_tile(ccs_batch *b, int group, int *tile_x, int *tile_y, int *ctas) {
+  if (!b || group < 0 || group >= (int)b->groups.size()) return CCS_ERR_ARG;
+  BATCH_TRY(b, cudaSetDevice(b->device));
+  const BatchGroup &g = b->groups[group];
+  StageTile t{};
+  if (g.lane == CCS_MIXED)
+    BATCH_TRY(b, mixed_stage_tile(g.var, g.nwork, &t));
+  else
+    t = f64_stage_tile(g.var, g.nwork, g.grid);
+  if (tile_x) *tile_x = t.tx;
+  if (tile_y) *tile_y = t.ty;
+  if (ctas) *ctas = t.ctas;
   return CCS_OK;
 }
 

@@ -777,14 +777,24 @@ constexpr int f64_smem_bytes() {
 }
 
 template <class T>
-int f64_grid_for(int device) {
-  int sms = 0, per = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+int f64_resident() {  // CTAs on an SM
+  int per = 0;
   constexpr int smem = f64_smem_bytes<T>();
   cudaFuncSetAttribute(f64_stage_kernel<T>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, f64_stage_kernel<T>, T::NT, smem);
-  if (per < 1) per = 1;
-  return sms * per;
+  return per < 1 ? 1 : per;
+}
+
+template <class T>
+int f64_grid_for(int device) {
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  return sms * f64_resident<T>();
+}
+
+template <class T>
+StageTile f64_tile_of() {
+  return StageTile{T::TX, T::TY, f64_resident<T>()};
 }
 
 template <class T>
@@ -831,13 +841,18 @@ int f64_max_grid(int var, int device) {
 //   in two (16 x 8 cells) when there are at most three an SM: C64 54 -> 49, C96 84 -> 67
 //   (larger grids lose by the halo cells of the parts: C192 245 -> 260, C384 921 -> 985)
 // grid: the resident CTAs of whole items, two an SM.  64 x 4 items have no such parts.
+static int f64_parts(int var, int nwork, int grid) {
+  if (var == 2) return 1;
+#ifdef CCS_BOUNDS  // (the checked build reaches all three on small grids)
+  return nwork <= 12 ? 4 : nwork <= 24 ? 2 : 1;
+#else
+  return 4 * nwork <= grid ? 4 : 4 * nwork <= 3 * grid ? 2 : 1;
+#endif
+}
+
 cudaError_t launch_f64_stage(int var, const F64Stage *d_stages, const WorkItem *d_work, int nwork, int grid,
                              cudaStream_t s, bool chained) {
-#ifdef CCS_BOUNDS  // (the checked build reaches all three on small grids)
-  const int parts = nwork <= 12 ? 4 : nwork <= 24 ? 2 : 1;
-#else
-  const int parts = 4 * nwork <= grid ? 4 : 4 * nwork <= 3 * grid ? 2 : 1;
-#endif
+  const int parts = f64_parts(var, nwork, grid);
   switch (var) {
     case 1:
       if (parts == 4) return f64_launch_parts<F64S1>(d_stages, d_work, nwork, s, chained);
@@ -849,6 +864,13 @@ cudaError_t launch_f64_stage(int var, const F64Stage *d_stages, const WorkItem *
       if (parts == 2) return f64_launch_parts<F64H0>(d_stages, d_work, nwork, s, chained);
       return f64_launch<F64T0>(d_stages, d_work, nwork, grid, s, chained);
   }
+}
+
+StageTile f64_stage_tile(int var, int nwork, int grid) {
+  const int parts = f64_parts(var, nwork, grid);
+  if (parts == 4) return f64_tile_of<F64S0>();  // (F64S1 alike; so F64H1)
+  if (parts == 2) return f64_tile_of<F64H0>();
+  return var == 1 ? f64_tile_of<F64T1>() : var == 2 ? f64_tile_of<F64T2>() : f64_tile_of<F64T0>();
 }
 
 // Products of static metric terms, each in the order the operator forms it: sqrtG f,

@@ -135,6 +135,12 @@ constexpr int kMxStaging[MX_NVAR] = {kStageLoads, kStageLoads, kStageAsync, kSta
 cudaError_t launch_f64_stage(int var, const F64Stage *d_stages, const WorkItem *d_work, int nwork, int grid,
                              cudaStream_t s, bool chained = false);
 int f64_max_grid(int var, int device);
+// what a CTA of such a launch works on: a work item, or the part of one that the launch's
+// size selects; and how many of them an SM of the current device holds
+struct StageTile {
+  int tx, ty, ctas;
+};
+StageTile f64_stage_tile(int var, int nwork, int grid);
 // the derived metric arrays of MeshF64 (sqrtGf, rsqrtG, lamx, lamy: consecutive fields at out)
 cudaError_t launch_f64_mesh_products(const Layout &L, const MeshF64 &m, double *out, cudaStream_t s);
 
@@ -144,6 +150,7 @@ cudaError_t launch_mixed_stage(int var, bool central, bool ediss, const MixedSta
                                const WorkItem *d_work, int nwork, int grid, cudaStream_t s,
                                bool chained = false);
 int mixed_max_grid(int var, int device);
+cudaError_t mixed_stage_tile(int var, int nwork, StageTile *tile);
 cudaError_t launch_mixed_import(const Layout &L, const double *phi, const double *u, const double *v,
                                 double phibar, double inv_a2, StateMixed out, float *lohp, float *lou,
                                 float *lov, cudaStream_t s);

@@ -941,14 +941,24 @@ static_assert(kMxStaging[0] == kStageLoads && kMxStaging[1] == kStageLoads && kM
               "staging table");
 
 template <class T, int STG>
-int mx_grid_for(int device) {  // the WENO instance bounds the occupancy of all
-  int sms = 0, per = 0;
-  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+int mx_resident() {  // CTAs on an SM; the WENO instance bounds the occupancy of all
+  int per = 0;
   constexpr int smem = (int)sizeof(SmemMx<T>);
   cudaFuncSetAttribute(mixed_stage_kernel<T, false, false, STG>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
   cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per, mixed_stage_kernel<T, false, false, STG>, T::NT, smem);
-  if (per < 1) per = 1;
-  return sms * per;
+  return per < 1 ? 1 : per;
+}
+
+template <class T, int STG>
+int mx_grid_for(int device) {
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, device);
+  return sms * mx_resident<T, STG>();
+}
+
+template <class T, int STG>
+StageTile mx_tile_of() {
+  return StageTile{T::TX, T::TY, mx_resident<T, STG>()};
 }
 
 // nwork items, each of sx x sy tiles
@@ -989,21 +999,23 @@ int mixed_max_grid(int var, int device) {
 // CTA, alone on its SM: every phase is a chain of loads or of dependent operations.
 // Launches with few items therefore run in smaller tiles with shorter line segments and
 // fewer cells per thread, one CTA each:
-//   16 x 8, two faces a segment, while no SM holds more than three (about C100): C24 11.8
+//   16 x 8, two faces a segment, while no SM holds more than three (up to C96): C24 11.8
 //   -> 5.7 us a stage, C48 11.8 -> 6.7, C96 11.8 -> 7.7 (C128 10.8, C160 14.7)
-//   16 x 16, four faces a segment, while all of them are resident, six an SM (about C190):
+//   16 x 16, four faces a segment, while all of them are resident, six an SM (up to C192):
 //   C112 11.8 -> 9.6, C128 11.8 -> 9.7, C160 11.8 -> 10.8, C192 14.0 -> 13.3 (C208 15.4 ->
 //   17.9: the shorter segments compute a quarter more cells, and a second wave begins)
 // (both sides in unchained launches; chained, eight steps a graph and with the 16 x 8 tiles'
 // operands in flight before the wait: C24 4.6, C48 5.1, C96 6.7, C128 9.3, C192 12.8)
 // Same bits in every tile shape.
-cudaError_t launch_mixed_stage(int var, bool central, bool ediss, const MixedStage *d_stages,
-                               const WorkItem *d_work, int nwork, int grid, cudaStream_t s,
-                               bool chained) {
+enum { kWhole, kMid, kSmall };
+static cudaError_t mixed_parts(int var, int nwork, int *size) {
   const TileShape ts = kMxTiles[var];
   const int small = nwork * (ts.tx / MxS::TX) * (ts.ty / MxS::TY), mid = nwork * (ts.tx / MxM::TX) * (ts.ty / MxM::TY);
 #ifdef CCS_BOUNDS
-  const int most_small = 6, most_mid = 24;  // (the checked build reaches all three on small grids)
+  // the checked build reaches all three on small grids, the largest of which has 24 items of
+  // 32 x 32 cells (192 small parts, 96 mid) or 36 of 32 x 16 (144, 72), the others at most 6
+  // or 12 (48 small parts either way)
+  const int most_small = 48, most_mid = 72;
 #else
   int dev = 0, sms = 0;
   cudaError_t e = cudaGetDevice(&dev);
@@ -1011,18 +1023,47 @@ cudaError_t launch_mixed_stage(int var, bool central, bool ediss, const MixedSta
   if (e != cudaSuccess) return e;
   const int most_small = 3 * sms, most_mid = 6 * sms;
 #endif
-  if (small <= most_small)
-    return mx_launch_any<MxS, kStageAsync>(central, ediss, d_stages, d_work, nwork, ts.tx / MxS::TX, ts.ty / MxS::TY,
-                                           small, s, chained);
-  if (mid <= most_mid)
-    return mx_launch_any<MxM, kStageLoads>(central, ediss, d_stages, d_work, nwork, ts.tx / MxM::TX, ts.ty / MxM::TY,
-                                           mid, s, chained);
+  *size = small <= most_small ? kSmall : mid <= most_mid ? kMid : kWhole;
+  return cudaSuccess;
+}
+
+cudaError_t launch_mixed_stage(int var, bool central, bool ediss, const MixedStage *d_stages,
+                               const WorkItem *d_work, int nwork, int grid, cudaStream_t s,
+                               bool chained) {
+  int size = kWhole;
+  const cudaError_t e = mixed_parts(var, nwork, &size);
+  if (e != cudaSuccess) return e;
+  const TileShape ts = kMxTiles[var];
+  if (size == kSmall) {
+    const int sx = ts.tx / MxS::TX, sy = ts.ty / MxS::TY;
+    return mx_launch_any<MxS, kStageAsync>(central, ediss, d_stages, d_work, nwork, sx, sy, nwork * sx * sy, s, chained);
+  }
+  if (size == kMid) {
+    const int sx = ts.tx / MxM::TX, sy = ts.ty / MxM::TY;
+    return mx_launch_any<MxM, kStageLoads>(central, ediss, d_stages, d_work, nwork, sx, sy, nwork * sx * sy, s, chained);
+  }
   switch (var) {
     case 1: return mx_launch_any<MxT1, kStageLoads>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s, chained);
     case 2: return mx_launch_any<MxT0, kStageAsync>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s, chained);
     case 3: return mx_launch_any<MxT1, kStageAsync>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s, chained);
     default: return mx_launch_any<MxT0, kStageLoads>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s, chained);
   }
+}
+
+cudaError_t mixed_stage_tile(int var, int nwork, StageTile *tile) {
+  int size = kWhole;
+  const cudaError_t e = mixed_parts(var, nwork, &size);
+  if (e != cudaSuccess) return e;
+  if (size != kWhole)
+    *tile = size == kSmall ? mx_tile_of<MxS, kStageAsync>() : mx_tile_of<MxM, kStageLoads>();
+  else
+    switch (var) {
+      case 1: *tile = mx_tile_of<MxT1, kStageLoads>(); break;
+      case 2: *tile = mx_tile_of<MxT0, kStageAsync>(); break;
+      case 3: *tile = mx_tile_of<MxT1, kStageAsync>(); break;
+      default: *tile = mx_tile_of<MxT0, kStageLoads>(); break;
+    }
+  return cudaSuccess;
 }
 
 static int ew_grid(const Layout &L) {

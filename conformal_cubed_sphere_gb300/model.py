@@ -258,6 +258,14 @@ class Stepper:
         L.check(L.lib().ccs_get_variant(self.handle, C.byref(v), C.byref(tx), C.byref(ty)), "ccs_get_variant")
         return v.value, tx.value, ty.value
 
+    @property
+    def stage_tile(self):
+        """(tile_x, tile_y, CTAs an SM holds) of this handle's stage launches
+        (ccs_stage_tile): the variant's work item or the part of it that small grids run."""
+        t = [C.c_int() for _ in range(3)]
+        L.check(L.lib().ccs_stage_tile(self.handle, *map(C.byref, t)), "ccs_stage_tile", self.handle)
+        return tuple(x.value for x in t)
+
     def close(self):
         if self.handle:
             L.lib().ccs_destroy(self.handle)
@@ -376,6 +384,12 @@ class Batch:
         lane, var, mem = (C.c_int * n.value)(), (C.c_int * n.value)(), (C.c_int * n.value)()
         L.check(L.lib().ccs_batch_info(self.handle, C.byref(n), n.value, lane, var, mem), "ccs_batch_info")
         return n.value, [(lane[q], var[q], mem[q]) for q in range(n.value)]
+
+    def stage_tile(self, group: int = 0):
+        """Stepper.stage_tile of one group of info()."""
+        t = [C.c_int() for _ in range(3)]
+        self._check(L.lib().ccs_batch_stage_tile(self.handle, int(group), *map(C.byref, t)), "ccs_batch_stage_tile")
+        return tuple(x.value for x in t)
 
     @property
     def stream_ptr(self) -> int:

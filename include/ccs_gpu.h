@@ -192,6 +192,11 @@ int ccs_set_operator(ccs_handle *h, int op);
 int ccs_autotune(ccs_handle *h, int reps, int force, int *chosen, double *times_us);
 int ccs_set_variant(ccs_handle *h, int variant);
 int ccs_get_variant(ccs_handle *h, int *variant, int *tile_x, int *tile_y);
+/* What one CTA of the handle's stage launches works on: the variant's work item, or the
+ * part of one that a launch with few work items runs; ctas: how many an SM holds at once
+ * (any pointer may be NULL).  For a batch, those of group `group` (ccs_batch_info). */
+int ccs_stage_tile(ccs_handle *h, int *tile_x, int *tile_y, int *ctas);
+int ccs_batch_stage_tile(ccs_batch *b, int group, int *tile_x, int *tile_y, int *ctas);
 
 /* spatial_operator(stat(old), tend) (spatial_operators_mod.F90:13-181): the
  * tendencies of phiG, u, v of the current state, interior cells (halo and corner
