@@ -425,10 +425,22 @@ static int build_f64_lane(ccs_handle *h) {
                              cudaMemcpyHostToDevice, h->stream));
   int rc = build_work(h, kF64Tiles[h->var], &h->d_work, &h->nwork);
   if (rc) return rc;
-  h->grid = f64_max_grid(h->var, c.device);
+  h->grid = f64_max_grid(h->var, h->op != CCS_OP_WENO, c.device);
   CCS_TRY(h, cudaMalloc(&h->d_partials, 2 * kDiagBlocks * sizeof(double)));
   CCS_TRY(h, cudaStreamSynchronize(h->stream));
   return CCS_OK;
+}
+
+static void f64_drop_graphs(ccs_handle *h) {
+  if (h->g_step) cudaGraphExecDestroy(h->g_step);
+  if (h->g_step_sw) cudaGraphExecDestroy(h->g_step_sw);
+  if (h->g_steps) cudaGraphExecDestroy(h->g_steps);
+  h->g_step = h->g_step_sw = h->g_steps = nullptr;
+}
+
+// one launch of the handle's FP64 stage kernel over stage descriptor d
+static cudaError_t f64_launch(ccs_handle *h, const F64Stage *d, bool chained = false) {
+  return launch_f64_stage(h->var, h->op != CCS_OP_WENO, d, h->d_work, h->nwork, h->grid, h->stream, chained);
 }
 
 // enqueue one step; with_sw: the final stage also writes the sphere winds; first: the
@@ -437,8 +449,7 @@ static int f64_enqueue_step(ccs_handle *h, bool with_sw, bool first = true) {
   for (int k = 0; k < h->n_rk; k++) {
     const F64Stage *d = h->d_stages + ((k == h->n_rk - 1 && with_sw) ? h->n_rk : k);
     if (h->timing) CCS_TRY(h, cudaEventRecord(h->ev0, h->stream));
-    CCS_TRY(h, launch_f64_stage(h->var, d, h->d_work, h->nwork, h->grid, h->stream,
-                                (k > 0 || !first) && !h->timing));
+    CCS_TRY(h, f64_launch(h, d, (k > 0 || !first) && !h->timing));
     if (h->timing) {
       CCS_TRY(h, cudaEventRecord(h->ev1, h->stream));
       CCS_TRY(h, cudaEventSynchronize(h->ev1));
@@ -732,6 +743,9 @@ int ccs_set_operator(ccs_handle *h, int op) {
   if (op != CCS_OP_WENO && op != CCS_OP_CENTRAL2 && op != CCS_OP_CENTRAL4 && op != CCS_OP_CENTRAL6)
     return CCS_ERR_ARG;
   cudaSetDevice(h->cfg.device);
+  // (of the FP64 variants only the 64 x 4 tile has a kernel of its own for central operators)
+  const bool other_kernel =
+      (op != CCS_OP_WENO) != (h->op != CCS_OP_WENO) && h->cfg.precision == CCS_FP64 && h->var == 2;
   h->op = op;
   if (h->cfg.precision == CCS_MIXED) {
     // the stage descriptors exist once the state (and with it phibar) is set
@@ -739,10 +753,14 @@ int ccs_set_operator(ccs_handle *h, int op) {
   }
   for (F64Stage &s : h->h_stages) s.op = op;
   // the captured graphs read the descriptors from device memory: updating them in
-  // place (after the stream's pending steps) is all a change needs
+  // place (after the stream's pending steps) is all a change within one kernel needs
   CCS_TRY(h, cudaMemcpyAsync(h->d_stages, h->h_stages.data(), h->h_stages.size() * sizeof(F64Stage),
                              cudaMemcpyHostToDevice, h->stream));
   CCS_TRY(h, cudaStreamSynchronize(h->stream));
+  if (other_kernel) {
+    h->grid = f64_max_grid(h->var, op != CCS_OP_WENO, h->cfg.device);
+    f64_drop_graphs(h);
+  }
   return CCS_OK;
 }
 
@@ -751,7 +769,7 @@ int ccs_spatial_operator(ccs_handle *h, double *tp, double *tu, double *tv) {
   cudaSetDevice(h->cfg.device);
   if (h->cfg.precision == CCS_MIXED) return mixed_tend(h, tp, tu, tv);
   const F64Stage *d = h->d_stages + h->n_rk + 1;
-  CCS_TRY(h, launch_f64_stage(h->var, d, h->d_work, h->nwork, h->grid, h->stream));
+  CCS_TRY(h, f64_launch(h, d));
   void *const dst[3] = {tp, tu, tv};
   const void *const src[3] = {h->tend[0], h->tend[1], h->tend[2]};
   CCS_TRY(h, copy_field_runs(dst, src, 3, (size_t)h->L.field * sizeof(double), cudaMemcpyDeviceToHost, h->stream));
@@ -1300,11 +1318,8 @@ static int set_variant(ccs_handle *h, int var) {
     int rc = build_work(h, kF64Tiles[var], &h->d_work, &h->nwork);
     if (rc) return rc;
     h->var = var;
-    h->grid = f64_max_grid(var, dev);
-    if (h->g_step) cudaGraphExecDestroy(h->g_step);
-    if (h->g_step_sw) cudaGraphExecDestroy(h->g_step_sw);
-    if (h->g_steps) cudaGraphExecDestroy(h->g_steps);
-    h->g_step = h->g_step_sw = h->g_steps = nullptr;
+    h->grid = f64_max_grid(var, h->op != CCS_OP_WENO, dev);
+    f64_drop_graphs(h);
   }
   return CCS_OK;
 }
@@ -1325,7 +1340,7 @@ static int time_stages(ccs_handle *h, int reps, double *us) {
       MixedLane *M = h->mixed;
       return mixed_launch(h, M->d_stages + k, k > 0);
     }
-    return launch_f64_stage(h->var, h->d_stages + k, h->d_work, h->nwork, h->grid, h->stream, k > 0);
+    return f64_launch(h, h->d_stages + k, k > 0);
   };
   cudaError_t e = launch(0);  // warm-up
   for (int r = 0; r < reps && e == cudaSuccess; r++) {
@@ -1367,7 +1382,7 @@ extern "C" int ccs_stage_tile(ccs_handle *h, int *tile_x, int *tile_y, int *ctas
   if (h->cfg.precision == CCS_MIXED)
     CCS_TRY(h, mixed_stage_tile(h->mixed->var, h->mixed->nwork, &t));
   else
-    t = f64_stage_tile(h->var, h->nwork, h->grid);
+    t = f64_stage_tile(h->var, h->op != CCS_OP_WENO, h->nwork, h->grid);
   if (tile_x) *tile_x = t.tx;
   if (tile_y) *tile_y = t.ty;
   if (ctas) *ctas = t.ctas;
@@ -1456,8 +1471,8 @@ static int group_nvar(const BatchGroup &g) { return g.lane == CCS_FP64 ? F64_NVA
 static cudaError_t group_launch(BatchGroup &g, int k, bool with_sw, bool chained = false) {
   if (g.lane == CCS_FP64) {
     const int row = (k == g.n_rk - 1 && with_sw) ? g.n_rk : k;
-    return launch_f64_stage(g.var, (const F64Stage *)g.d_stages + (size_t)row * g.nmem, g.d_work, g.nwork, g.grid,
-                            g.stream, chained);
+    return launch_f64_stage(g.var, g.central, (const F64Stage *)g.d_stages + (size_t)row * g.nmem, g.d_work, g.nwork,
+                            g.grid, g.stream, chained);
   }
   return launch_mixed_stage(g.var, g.central, g.ediss, (const MixedStage *)g.d_stages + (size_t)k * g.nmem,
                             g.d_work, g.nwork, g.grid, g.stream, chained);
@@ -1486,7 +1501,7 @@ static int group_set_var(ccs_batch *b, BatchGroup &g, int var) {
   BATCH_TRY(b, cudaMemcpy(g.d_work, work.data(), work.size() * sizeof(WorkItem), cudaMemcpyHostToDevice));
   g.nwork = (int)work.size();
   g.var = var;
-  g.grid = g.lane == CCS_FP64 ? f64_max_grid(var, b->device) : mixed_max_grid(var, b->device);
+  g.grid = g.lane == CCS_FP64 ? f64_max_grid(var, g.central, b->device) : mixed_max_grid(var, b->device);
   return CCS_OK;
 }
 
@@ -1695,7 +1710,7 @@ extern "C" int ccs_batch_stage_tile(ccs_batch *b, int group, int *tile_x, int *t
   if (g.lane == CCS_MIXED)
     BATCH_TRY(b, mixed_stage_tile(g.var, g.nwork, &t));
   else
-    t = f64_stage_tile(g.var, g.nwork, g.grid);
+    t = f64_stage_tile(g.var, g.central, g.nwork, g.grid);
   if (tile_x) *tile_x = t.tx;
   if (tile_y) *tile_y = t.ty;
   if (ctas) *ctas = t.ctas;

@@ -40,9 +40,11 @@ constexpr int NSING = 6;
 
 // A tile of TX x TY cells worked on by NT threads, CTAS of them resident on an SM; phase
 // 3 maps one thread to one cell.  The tile is one of the PX / TX x PY / TY parts of a work
-// item of PX x PY cells (the item itself unless a launch is split).
-template <int TX_, int TY_, int NT_, int CTAS_, int PX_ = TX_, int PY_ = TY_>
+// item of PX x PY cells (the item itself unless a launch is split).  FACES: with the face
+// phases and their shared memory; a tile without runs central-difference operators only.
+template <int TX_, int TY_, int NT_, int CTAS_, int PX_ = TX_, int PY_ = TY_, bool FACES_ = true>
 struct F64Tile {
+  static constexpr bool FACES = FACES_;
   static constexpr int TX = TX_, TY = TY_, NC = TX * TY, NT = NT_, CTAS = CTAS_;
   static constexpr int SX = PX_ / TX, SY = PY_ / TY, PX = PX_, PY = PY_;
   static constexpr int RX = TX + 6, RY = TY + 6, RN = RX * RY;
@@ -50,7 +52,8 @@ struct F64Tile {
   // cells of the lines through the tile: rows of RX cells, columns of RY
   static constexpr int NLX = TY * RX, NLY = RY * TX;
   static constexpr int NSCR_F = (NSING + 2) * (NLX + NLY), NSCR_E = NSING * RN + 2 * (NLX + NLY);
-  static constexpr int NSCR = NSCR_F > NSCR_E ? NSCR_F : NSCR_E;
+  static constexpr int NSCR = !FACES ? 3 * NC : NSCR_F > NSCR_E ? NSCR_F : NSCR_E;
+  static constexpr int NREC = FACES ? NF : 1;
 };
 }  // namespace
 
@@ -326,9 +329,10 @@ struct Smem {
   double phit[T::RN], phitG[T::RN], E[T::RN], Fx[T::RN], Fy[T::RN], uC[T::RN], vC[T::RN], u[T::RN], v[T::RN];
   // face values: sums of the two sides of the flux and E, difference of phitG's (and of
   // the wind's: E dissipation); then the Rusanov fluxes of phiG and E in the first two
-  double rec[4][T::NF];
+  double rec[4][T::NREC];
   // per-cell products of the fields of one pass: either fields of their own on the rows
-  // and columns, or one field on the halo'd tile with curvatures on rows and columns
+  // and columns, or one field on the halo'd tile with curvatures on rows and columns; then
+  // the cells' new values for the push
   double scr[T::NSCR];
   F64Stage st;  // the work item's stage descriptor
 };
@@ -563,7 +567,7 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
 
     // ---- phase 2: face reconstructions (weno, :183-277) ---------------------
     // (the central-difference operators have no faces: straight to phase 3)
-    if (op == CCS_OP_WENO) {
+    if constexpr (T::FACES) if (op == CCS_OP_WENO) {
     reconstruct<T, false, false>(S, f, S.Fx, S.Fy, S.rec[0], nx, ny, slow);
     reconstruct<T, true, false>(S, f, S.E, S.E, S.rec[1], nx, ny, slow);
     reconstruct<T, true, true>(S, f, S.phitG, S.phitG, S.rec[2], nx, ny, slow);
@@ -635,7 +639,7 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
         const double a11 = __ldg(st.m.aig11 + c), a12 = __ldg(st.m.aig12 + c), a21 = __ldg(st.m.aig21 + c),
                      a22 = __ldg(st.m.aig22 + c);
         double dfluxdx, dEdx, dvdx, dfluxdy, dEdy, dudy;
-        if (op == CCS_OP_WENO) {
+        if (T::FACES && op == CCS_OP_WENO) {
           const double *FF = S.rec[0], *EF = S.rec[1];
           const int xl = lj * (TX + 1) + li, xr = xl + 1;
           const int yb = NFX + lj * TX + li, yt = yb + TX;
@@ -764,6 +768,10 @@ namespace {
 using F64T0 = F64Tile<32, 8, 384, 2>;
 using F64T1 = F64Tile<16, 16, 384, 2>;
 using F64T2 = F64Tile<64, 4, 384, 1>;
+// 64 x 4 items of the central operators: the face phases' shared memory leaves room for one
+// CTA an SM (the other tiles hold two); without it two fit (fourth-order operator: C384 306 ->
+// 243 us a stage, C192 79 -> 67, C96 28.8 -> 24.5; three of 256 threads 256, 65, 26.1)
+using F64C2 = F64Tile<64, 4, 384, 2, 64, 4, false>;
 // parts of 16 x 8 cells, three CTAs an SM
 using F64H0 = F64Tile<16, 8, 288, 3, 32, 8>;
 using F64H1 = F64Tile<16, 8, 288, 3, 16, 16>;
@@ -823,13 +831,14 @@ cudaError_t f64_launch_parts(const F64Stage *d_stages, const WorkItem *d_work, i
 static_assert(F64T0::TX == kF64Tiles[0].tx && F64T0::TY == kF64Tiles[0].ty, "tile table");
 static_assert(F64T1::TX == kF64Tiles[1].tx && F64T1::TY == kF64Tiles[1].ty, "tile table");
 static_assert(F64T2::TX == kF64Tiles[2].tx && F64T2::TY == kF64Tiles[2].ty, "tile table");
+static_assert(F64C2::TX == kF64Tiles[2].tx && F64C2::TY == kF64Tiles[2].ty, "tile table");
 
 }  // namespace
 
-int f64_max_grid(int var, int device) {
+int f64_max_grid(int var, bool central, int device) {
   switch (var) {
     case 1: return f64_grid_for<F64T1>(device);
-    case 2: return f64_grid_for<F64T2>(device);
+    case 2: return central ? f64_grid_for<F64C2>(device) : f64_grid_for<F64T2>(device);
     default: return f64_grid_for<F64T0>(device);
   }
 }
@@ -850,15 +859,17 @@ static int f64_parts(int var, int nwork, int grid) {
 #endif
 }
 
-cudaError_t launch_f64_stage(int var, const F64Stage *d_stages, const WorkItem *d_work, int nwork, int grid,
-                             cudaStream_t s, bool chained) {
+cudaError_t launch_f64_stage(int var, bool central, const F64Stage *d_stages, const WorkItem *d_work, int nwork,
+                             int grid, cudaStream_t s, bool chained) {
   const int parts = f64_parts(var, nwork, grid);
   switch (var) {
     case 1:
       if (parts == 4) return f64_launch_parts<F64S1>(d_stages, d_work, nwork, s, chained);
       if (parts == 2) return f64_launch_parts<F64H1>(d_stages, d_work, nwork, s, chained);
       return f64_launch<F64T1>(d_stages, d_work, nwork, grid, s, chained);
-    case 2: return f64_launch<F64T2>(d_stages, d_work, nwork, grid, s, chained);
+    case 2:
+      if (central) return f64_launch<F64C2>(d_stages, d_work, nwork, grid, s, chained);
+      return f64_launch<F64T2>(d_stages, d_work, nwork, grid, s, chained);
     default:
       if (parts == 4) return f64_launch_parts<F64S0>(d_stages, d_work, nwork, s, chained);
       if (parts == 2) return f64_launch_parts<F64H0>(d_stages, d_work, nwork, s, chained);
@@ -866,11 +877,12 @@ cudaError_t launch_f64_stage(int var, const F64Stage *d_stages, const WorkItem *
   }
 }
 
-StageTile f64_stage_tile(int var, int nwork, int grid) {
+StageTile f64_stage_tile(int var, bool central, int nwork, int grid) {
   const int parts = f64_parts(var, nwork, grid);
   if (parts == 4) return f64_tile_of<F64S0>();  // (F64S1 alike; so F64H1)
   if (parts == 2) return f64_tile_of<F64H0>();
-  return var == 1 ? f64_tile_of<F64T1>() : var == 2 ? f64_tile_of<F64T2>() : f64_tile_of<F64T0>();
+  if (var == 2) return central ? f64_tile_of<F64C2>() : f64_tile_of<F64T2>();
+  return var == 1 ? f64_tile_of<F64T1>() : f64_tile_of<F64T0>();
 }
 
 // Products of static metric terms, each in the order the operator forms it: sqrtG f,

@@ -132,15 +132,16 @@ constexpr TileShape kMxTiles[MX_NVAR] = {{32, 32}, {32, 16}, {32, 32}, {32, 16}}
 constexpr int kMxStaging[MX_NVAR] = {kStageLoads, kStageLoads, kStageAsync, kStageAsync};
 
 // kernel launchers (return cudaGetLastError()); `var` indexes the tile tables
-cudaError_t launch_f64_stage(int var, const F64Stage *d_stages, const WorkItem *d_work, int nwork, int grid,
-                             cudaStream_t s, bool chained = false);
-int f64_max_grid(int var, int device);
+// (central: every stage in d_stages uses a central-difference operator, else WENO-Z)
+cudaError_t launch_f64_stage(int var, bool central, const F64Stage *d_stages, const WorkItem *d_work, int nwork,
+                             int grid, cudaStream_t s, bool chained = false);
+int f64_max_grid(int var, bool central, int device);
 // what a CTA of such a launch works on: a work item, or the part of one that the launch's
 // size selects; and how many of them an SM of the current device holds
 struct StageTile {
   int tx, ty, ctas;
 };
-StageTile f64_stage_tile(int var, int nwork, int grid);
+StageTile f64_stage_tile(int var, bool central, int nwork, int grid);
 // the derived metric arrays of MeshF64 (sqrtGf, rsqrtG, lamx, lamy: consecutive fields at out)
 cudaError_t launch_f64_mesh_products(const Layout &L, const MeshF64 &m, double *out, cudaStream_t s);
 
