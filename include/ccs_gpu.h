@@ -180,14 +180,16 @@ int ccs_set_operator(ccs_handle *h, int op);
  * and 3: 32x16 with asynchronous copies (the raw inputs of all of a thread's cells
  * go into shared memory at once, then are derived in place).  Every variant
  * computes the same per-cell arithmetic, so results do not depend on the choice; a
- * launch with few work items runs smaller parts of them, whatever the variant.  ccs_autotune times the handle's RK stages before the last one (they write
- * only stage scratch, so the state is unchanged), `reps` rounds with each variant
- * after one warm-up launch, and keeps the fastest mean stage time; the choice is cached per (device, lane, N,
- * halo) for the process, and later calls with force = 0 reuse it without timing.
- * The state must be set first.  chosen (may be NULL) receives the variant,
- * times_us (may be NULL, CCS_MAX_VARIANTS entries) the mean launch times in
- * microseconds (0 where nothing was timed).  A batch groups its members by
- * variant, so tune members before ccs_batch_create. */
+ * launch with few work items runs smaller parts of them, whatever the variant
+ * (ccs_stage_tile).  ccs_autotune times the handle's RK stages before the last one (they
+ * write only stage scratch, so the state is unchanged), `reps` rounds with each variant
+ * after one warm-up launch, and keeps the fastest mean stage time; variants that run the
+ * same parts are timed once, and of these the one that is fastest whole is kept.  The
+ * choice is cached per (device, lane, N, halo) for the process, and later calls with
+ * force = 0 reuse it without timing.  The state must be set first.  chosen (may be NULL)
+ * receives the variant, times_us (may be NULL, CCS_MAX_VARIANTS entries) the mean launch
+ * times in microseconds (0 where nothing was timed).  A batch takes the variant of its
+ * largest member in each group, so tune members before ccs_batch_create. */
 #define CCS_MAX_VARIANTS 4
 int ccs_autotune(ccs_handle *h, int reps, int force, int *chosen, double *times_us);
 int ccs_set_variant(ccs_handle *h, int variant);
