@@ -276,11 +276,13 @@ static int build_mesh(ccs_handle *h, const ccs_mesh_view *mv) {
   const Layout &L = h->L;
   const size_t nref = (size_t)L.nh * L.nh * 6;
   const size_t nf = (size_t)L.field;
-  // FP64 arrays: sqrtG phis f ig11 ig12 ig21 ig22 aig11..22 gia11..22 from the host, and
-  // sqrtGf rsqrtG lamx lamy formed from them on the device
-  constexpr int na = 15, nd = 4;
-  CCS_TRY(h, cudaMalloc(&dm->buf64, (na + nd) * nf * sizeof(double)));
-  CCS_TRY(h, cudaMemsetAsync(dm->buf64, 0, (na + nd) * nf * sizeof(double), h->stream));
+  // FP64 arrays: sqrtG phis f ig11 ig12 ig21 ig22 aig11..22 gia11..22 from the host; for the
+  // FP64 lane, whose stage kernel alone reads them, also sqrtGf rsqrtG lamx lamy, formed from
+  // those on the device
+  constexpr int na = 15;
+  const int nd = h->cfg.precision == CCS_FP64 ? 4 : 0;
+  CCS_TRY(h, cudaMalloc(&dm->buf64, (size_t)(na + nd) * nf * sizeof(double)));
+  CCS_TRY(h, cudaMemsetAsync(dm->buf64, 0, (size_t)(na + nd) * nf * sizeof(double), h->stream));
   std::vector<double> tmp(na * nref, 0.);
   double *t[na];
   for (int k = 0; k < na; k++) t[k] = tmp.data() + k * nref;
@@ -310,8 +312,10 @@ static int build_mesh(ccs_handle *h, const ccs_mesh_view *mv) {
   dm->m64.ig11 = b + 3 * nf; dm->m64.ig12 = b + 4 * nf; dm->m64.ig21 = b + 5 * nf; dm->m64.ig22 = b + 6 * nf;
   dm->m64.aig11 = b + 7 * nf; dm->m64.aig12 = b + 8 * nf; dm->m64.aig21 = b + 9 * nf; dm->m64.aig22 = b + 10 * nf;
   dm->m64.gia11 = b + 11 * nf; dm->m64.gia12 = b + 12 * nf; dm->m64.gia21 = b + 13 * nf; dm->m64.gia22 = b + 14 * nf;
-  dm->m64.sqrtGf = b + 15 * nf; dm->m64.rsqrtG = b + 16 * nf; dm->m64.lamx = b + 17 * nf; dm->m64.lamy = b + 18 * nf;
-  CCS_TRY(h, launch_f64_mesh_products(L, dm->m64, b + 15 * nf, h->stream));
+  if (nd) {
+    dm->m64.sqrtGf = b + 15 * nf; dm->m64.rsqrtG = b + 16 * nf; dm->m64.lamx = b + 17 * nf; dm->m64.lamy = b + 18 * nf;
+    CCS_TRY(h, launch_f64_mesh_products(L, dm->m64, b + 15 * nf, h->stream));
+  }
   std::vector<int32_t> push;
   if (!build_push_table(L, push)) {
     h->err = "ghost tables are inconsistent";

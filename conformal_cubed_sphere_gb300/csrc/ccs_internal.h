@@ -60,7 +60,7 @@ struct MeshF64 {
   const double *ig11, *ig12, *ig21, *ig22;
   const double *aig11, *aig12, *aig21, *aig22;
   const double *gia11, *gia12, *gia21, *gia22;
-  // products of static metric terms, formed once in the order the operator forms them:
+  // (FP64 lane only) products of static metric terms, formed once in the operator's order:
   // sqrtG f; RN(1 / sqrtG); and (IG11(i+1,j) + IG11(i,j)) / 2 of the x-face right of cell
   // (i, j), (IG22(i,j+1) + IG22(i,j)) / 2 of the y-face above it, both at the cell's index
   const double *sqrtGf, *rsqrtG, *lamx, *lamy;
