@@ -211,6 +211,10 @@ static cudaError_t copy_field_runs(void *const *dst, const void *const *src, int
 static int validate_config(const ccs_config *c) {
   if (!c) return CCS_ERR_ARG;
   if (c->N < 1 || c->N > 8192 || c->halo < 3 || c->halo > c->N) return CCS_ERR_ARG;
+  // the push table and the mixed lane's stage kernel hold cell offsets in 32 bits (a field of
+  // 2^31 cells would take a handle more than 500 GB)
+  const int64_t nh = (int64_t)c->N + 2 * c->halo;
+  if (6 * nh * ((nh + 3) / 4 * 4) > INT32_MAX) return CCS_ERR_ARG;
   if (c->scheme != CCS_RK4 && c->scheme != CCS_RK3_TVD) return CCS_ERR_ARG;
   if (c->precision != CCS_FP64 && c->precision != CCS_MIXED) return CCS_ERR_ARG;
   if (c->e_dissipation != CCS_EDISS_ZERO && c->e_dissipation != CCS_EDISS_RECONSTRUCT) return CCS_ERR_ARG;

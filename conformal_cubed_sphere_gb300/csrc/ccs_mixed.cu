@@ -706,7 +706,7 @@ mixed_stage_kernel(const MixedStage *__restrict__ stages, const WorkItem *__rest
       const float phibar = st.phibar, ha2 = 0.5f * st.a2;
       const float *ihp = st.in.hp, *iu = st.in.u, *iv = st.in.v;
       const MeshMixed m = st.m;
-      // offsets fit 32 bits: a field has 6 (N + 2 h)^2 cells, N at most 8192
+      // offsets fit 32 bits (validate_config sees to it)
       const int pan = (int)L.panel * p, origin = (int)L.idx(i0 - 3, j0 - 3, 0), pitch = L.pitch;
       // A cell that is not there (corner block, beyond the halo) is skipped by a branch
       // (BRANCH), or reads the panel's first cell and drops it.
