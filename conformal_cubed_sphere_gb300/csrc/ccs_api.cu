@@ -575,6 +575,25 @@ int ccs_selftest_div_pairs(const double *a, const double *b, int64_t n, double *
   return rc;
 }
 
+int ccs_selftest_integer(int what, const double *a, const double *b, int64_t n, double *fast, double *ieee) {
+  if (!a || !b || n <= 0 || !fast || !ieee || what < 0 || what > CCS_CHECK_RECONSTRUCTION) return CCS_ERR_ARG;
+  if (what == CCS_CHECK_RECONSTRUCTION && n % 5 != 0) return CCS_ERR_ARG;
+  int ndev = 0;
+  if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev < 1) return CCS_ERR_NODEVICE;
+  cudaSetDevice(0);
+  double *buf = nullptr;  // a, b, then both results
+  const size_t bytes = n * sizeof(double);
+  if (cudaMalloc(&buf, 4 * bytes) != cudaSuccess) return CCS_ERR_NOMEM;
+  const bool ok = cudaMemcpy(buf, a, bytes, cudaMemcpyHostToDevice) == cudaSuccess &&
+                  cudaMemcpy(buf + n, b, bytes, cudaMemcpyHostToDevice) == cudaSuccess &&
+                  cudaMemset(buf + 2 * n, 0, 2 * bytes) == cudaSuccess &&
+                  launch_integer_check(what, buf, buf + n, n, buf + 2 * n, 0) == cudaSuccess &&
+                  cudaMemcpy(fast, buf + 2 * n, bytes, cudaMemcpyDeviceToHost) == cudaSuccess &&
+                  cudaMemcpy(ieee, buf + 3 * n, bytes, cudaMemcpyDeviceToHost) == cudaSuccess;
+  cudaFree(buf);
+  return ok ? CCS_OK : CCS_ERR_CUDA;
+}
+
 const char *ccs_strerror(int status) {
   switch (status) {
     case CCS_OK: return "ok";

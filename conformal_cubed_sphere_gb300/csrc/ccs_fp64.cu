@@ -57,12 +57,11 @@ struct F64Tile {
 };
 }  // namespace
 
-// x / b for a divisor fixed in advance — the constants 3, 6, 12 of the reference
-// (x/3., x/6., A*A*13./12.) and a grid's dx, dy, 60 dx, 60 dy — correctly rounded:
-// q0 = RN(x y) with y = RN(1/b), the remainder
-// r = x - q0 b is exact in one FMA, and q0 + r y rounded once is RN(x / b)
-// (Markstein's correction, IBM J. Res. Dev. 34(1), 1990) when the quotient does not
-// underflow.  Where the correction does not apply, q0 is already the IEEE result: a
+// x / b for the constants 3, 6, 12 of the reference (x/3., x/6., A*A*13./12.) in tiles
+// outside the integer arithmetic's window, correctly rounded: q0 = RN(x y) with
+// y = RN(1/b), the remainder r = x - q0 b is exact in one FMA, and q0 + r y rounded once is
+// RN(x / b) (Markstein's correction, IBM J. Res. Dev. 34(1), 1990) when the quotient does
+// not underflow.  Where the correction does not apply, q0 is already the IEEE result: a
 // zero dividend keeps its sign, an infinite one stays infinite (the remainder would
 // be inf - inf = NaN) and a NaN stays NaN.  The GPU test suite checks this against
 // IEEE division.
@@ -751,6 +750,65 @@ __global__ void div_pairs_check_kernel(const double *__restrict__ a, const doubl
 cudaError_t launch_div_pairs_check(const double *a, const double *b, int64_t n, double *out, cudaStream_t s) {
   div_pairs_check_kernel<<<1024, 256, 0, s>>>(a, b, n, out);
   return cudaGetLastError();
+}
+
+// test support: out[k] = what the stage kernel computes with the integer routines, out[n + k]
+// = the IEEE operations it stands for (CCS_CHECK_*)
+__global__ void integer_check_kernel(int what, const double *__restrict__ a, const double *__restrict__ b, int64_t n,
+                                     double *__restrict__ out) {
+  using namespace softfp;
+  for (int64_t k = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; k < n; k += (int64_t)gridDim.x * blockDim.x) {
+    const double x = a[k], y = b[k];
+    double fast = 0., ieee = 0.;
+    switch (what) {
+      case CCS_CHECK_MUL: fast = round_double(mul(unpack(x), unpack(y))); ieee = x * y; break;
+      case CCS_CHECK_MUL_UNPACKED: fast = pack(round_unp(mul(unpack(x), unpack(y)))); ieee = x * y; break;
+      case CCS_CHECK_DIV: fast = round_double(div(unpack(x), divisor(unpack(y)))); ieee = x / y; break;
+      case CCS_CHECK_DIV_UNPACKED: fast = pack(round_unp(div(unpack(x), divisor(unpack(y))))); ieee = x / y; break;
+      case CCS_CHECK_ONE_PLUS_DIV:
+        fast = pack(round_unp(one_plus(div(unpack(x), divisor(unpack(y))))));
+        ieee = 1. + x / y;
+        break;
+      case CCS_CHECK_ADD: fast = pack(round_unp(add(unpack(x), unpack(y)))); ieee = x + y; break;
+      case CCS_CHECK_SQRT: fast = square_root(unpack(x)); ieee = sqrt(x); break;
+      case CCS_CHECK_CURVATURE: fast = curvature(x); ieee = x * x * 13. / 12.; break;
+      case CCS_CHECK_GRID_DIV: {
+        Divisor d = divisor(unpack(y));
+        if (!(y >= 0x1p-400 && y < 0x1p300)) d.y = 0u;  // (as the host prepares a grid's)
+        fast = div_by(x, d, y);
+        ieee = x / y;
+        break;
+      }
+      case CCS_CHECK_DIV6: fast = div_by6(x); ieee = x / 6.; break;
+      case CCS_CHECK_HALF: fast = half_of(x); ieee = 0.5 * x; break;
+    }
+    out[k] = fast;
+    out[n + k] = ieee;
+  }
+}
+
+// the same of one whole reconstruction: window k is a[5 k .. 5 k + 4]
+__global__ void side_check_kernel(const double *__restrict__ a, int64_t n, F64Ops f, double *__restrict__ out) {
+  const int64_t m = n / 5;
+  for (int64_t k0 = blockIdx.x * (int64_t)blockDim.x; k0 < m; k0 += (int64_t)gridDim.x * blockDim.x) {
+    const int64_t k = k0 + threadIdx.x, w = k < m ? k : m - 1;  // (whole warps, for the votes)
+    double Q[5], G[NSING * 5], ga[3];
+    for (int q = 0; q < 5; q++) Q[q] = a[5 * w + q];
+    for (int q = 0; q < 5; q++) store_singles(f, G + q, 5, Q[q]);
+    for (int q = 0; q < 3; q++) ga[q] = curvature(f.add(fma(-2., Q[q + 1], Q[q]), Q[q + 2]));
+    const double fast = side(f, 0xffffffffu, Q + 2, 1, G + 2, 5, 1, ga + 1, 1);
+    const double ieee = weno5z(Q[0], Q[1], Q[2], Q[3], Q[4]);
+    if (k < m) {
+      out[k] = fast;
+      out[n + k] = ieee;
+    }
+  }
+}
+
+cudaError_t launch_integer_check(int what, const double *a, const double *b, int64_t n, double *out, cudaStream_t s) {
+  if (what == CCS_CHECK_RECONSTRUCTION)
+    return launch_stage(side_check_kernel, 1024, 256, 0, s, false, a, n, F64Ops{1., -0.}, out);
+  return launch_stage(integer_check_kernel, 1024, 256, 0, s, false, what, a, b, n, out);
 }
 
 unsigned long long f64_bounds_take() { return bounds_take_tu(); }

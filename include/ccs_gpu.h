@@ -288,19 +288,33 @@ int ccs_ghost_map(int N, int halo, int64_t *src_index);
  * with CUDA events on the handle's stream when timing is enabled. */
 int ccs_timing(ccs_handle *h, int enable, int reset, double *kernel_ms, int64_t *launches);
 
-/* Self-check of the FP64 lane's division by the constants 3, 6 and 12: for each
- * x[k] the device computes the correctly rounded quotient the kernels use (fast[k])
- * and the IEEE quotient x[k] / b (ieee[k]); they must agree bit for bit.  Runs on
- * device 0 with temporary buffers. */
+/* Self-check of the FP64 lane's division by the constants 3, 6 and 12 outside the integer
+ * arithmetic's window: for each x[k] the device computes the correctly rounded quotient the
+ * kernels use there (fast[k]) and the IEEE quotient x[k] / b (ieee[k]); they must agree bit
+ * for bit.  Runs on device 0 with temporary buffers. */
 int ccs_selftest_div(const double *x, int64_t n, double b, double *fast, double *ieee);
 
-/* Self-check of the FP64 lane's division by a divisor several quotients share (the
- * WENO-Z weights alpha_k / sum(alpha)): for each pair the device computes the
- * quotient the kernels use, from the divisor's IEEE reciprocal and one FMA
- * correction (fast[k]), and the IEEE quotient a[k] / b[k] (ieee[k]); they must agree
- * bit for bit when the quotient is a normal number.  Runs on device 0 with temporary
- * buffers. */
+/* Self-check of the division by a divisor several quotients share (the WENO-Z weights
+ * alpha_k / sum(alpha) outside that window): for each pair the device computes the quotient
+ * the kernels use there, from the divisor's IEEE reciprocal and one FMA correction
+ * (fast[k]), and the IEEE quotient a[k] / b[k] (ieee[k]); they must agree bit for bit when
+ * the quotient is a normal number.  Runs on device 0 with temporary buffers. */
 int ccs_selftest_div_pairs(const double *a, const double *b, int64_t n, double *fast, double *ieee);
+
+/* Self-check of the FP64 lane's arithmetic on the integer pipes, as the device runs it:
+ * fast[k] from the integer routines, ieee[k] from the IEEE operations they stand for, to be
+ * equal bit for bit.  For positive a, b in [2^-200, 2^200): a b and a / b (each rounded to a
+ * double or kept unpacked), 1 + a / b, a + b and sqrt(a).  For any a of magnitude in that
+ * range or zero: (a a 13) / 12.  For any a, and b > 0: a / b as by a grid's dx, a / 6, a / 2.
+ * CCS_CHECK_RECONSTRUCTION: a[5 k .. 5 k + 4], zero or of magnitude in the range, are the
+ * cells of one WENO-Z reconstruction, n a multiple of 5, results in the first n / 5
+ * entries.  Runs on device 0 with temporary buffers. */
+enum {
+  CCS_CHECK_MUL, CCS_CHECK_MUL_UNPACKED, CCS_CHECK_DIV, CCS_CHECK_DIV_UNPACKED, CCS_CHECK_ONE_PLUS_DIV,
+  CCS_CHECK_ADD, CCS_CHECK_SQRT, CCS_CHECK_CURVATURE, CCS_CHECK_GRID_DIV, CCS_CHECK_DIV6, CCS_CHECK_HALF,
+  CCS_CHECK_RECONSTRUCTION
+};
+int ccs_selftest_integer(int what, const double *a, const double *b, int64_t n, double *fast, double *ieee);
 
 /* Bounds-checked build (libccs_gpu.so built with -DCCS_BOUNDS, build.build_bounds):
  * the kernels check their array indices and skip, instead of performing, any access
