@@ -219,6 +219,15 @@ __device__ __forceinline__ double half_of(double x) {
   return 0.5 * x;
 }
 
+// 2 x by its exponent; zeros, subnormals, infinities, NaNs and values whose double
+// overflows take the FP64 multiplication.  (fma(2, x, a) would not overflow where the
+// reference's 2 x does.)
+__device__ __forceinline__ double twice(double x) {
+  const uint32_t h = softfp::hi32(softfp::bits_of(x)), e = h & 0x7ff00000u;
+  if (e - 0x00100000u < 0x7fd00000u) return __hiloint2double((int)(h + 0x00100000u), __double2loint(x));
+  return 2. * x;
+}
+
 // Whether the integer arithmetic of the reconstructions covers a field value: zero or
 // of magnitude in [2^-200, 2^200).  Differences of such values are zero or at least
 // 2^-253, so the smoothness indicators lie in {0} or [2^-510, 2^410], the weights in
@@ -669,7 +678,7 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
           double n[3];
           if (kind == K_RK4_2)
 #pragma unroll
-            for (int q = 0; q < 3; q++) ac[q] = fma(2., t[q], ac[q]);
+            for (int q = 0; q < 3; q++) ac[q] = f.add(ac[q], twice(t[q]));
 #pragma unroll
           for (int q = 0; q < 3; q++) {
             if (kind == K_RK4_4)

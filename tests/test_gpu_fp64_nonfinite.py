@@ -41,3 +41,32 @@ def test_wave_speed_that_is_not_finite(value, ediss, entry):
     im = mesh.interior_mask()
     bad = [_same(a, b, im, q) for q, (a, b) in enumerate(zip(g.spatial_operator(), o.spatial_operator()))]
     assert bad[0] > 0 and max(bad[1:]) > 0  # (phiG, and the wind across the face)
+
+
+@pytest.mark.parametrize("seed", range(4))
+def test_doubled_tendencies_that_overflow(seed):
+    """RK4 adds 2 k2 to k1: where k2 is beyond 2^1023 the reference's product is infinite,
+    whatever k1 is.  A state of huge phiG over a huge sqrtG (so that the depth stays small
+    and the wind moderate) has such cells with k1 of the other sign."""
+    mesh, s, dt = seeded_case(16, 3, seed=3 + seed, oro=False)
+    mesh = copy.copy(mesh)
+    mesh.sqrtG, mesh.f, dt = mesh.sqrtG * 2.0 ** 975, mesh.f * 0, 1.0
+    for k in ("u", "v", "uC", "vC"):
+        s[k] *= 1e5
+    rng = np.random.default_rng(seed)
+    s["phi"][:] = 1.0
+    s["phiG"][:] = 2.0 ** 1021 * rng.uniform(-1, 1, size=mesh.ncell)
+    o = O.Oracle.from_mesh(mesh, operator=L.CCS_OP_CENTRAL2)
+    o.set_state(s.arrays)
+    o.rk4_once(dt)
+    im, m = mesh.interior_mask(), ~mesh.corner_mask()
+    k1, k2 = (o.get_tend(q)[0][im] for q in (-1, -2))
+    with np.errstate(all="ignore"):
+        cells = np.isinf(k1 + 2 * k2) & (np.abs(k1 / 4 + k2 / 2) < 2.0 ** 1021.9)
+    assert cells.sum() > 0
+    g = M.Stepper(mesh, dt, precision="fp64", operator=L.CCS_OP_CENTRAL2)
+    g.set_state(s)
+    g.step(1)
+    a, b = g.get_state(), o.get_state(1)
+    for k in ("phiG", "u", "v"):
+        _same(a[k], b[k], m, k)
