@@ -122,10 +122,13 @@ __device__ __forceinline__ double weno5z(double Qim2, double Qim1, double Qi, do
   long long mn = __double_as_longlong(be0);
   if (__double_as_longlong(be1) < mn) mn = __double_as_longlong(be1);
   if (__double_as_longlong(be2) < mn) mn = __double_as_longlong(be2);
+  // a comparison with a NaN (of betas that overflow, or of a cell that is not finite) is
+  // false; with the taus numbers, the betas are
+  const bool numbers = t40 <= 0x7ff0000000000000LL && t41 <= 0x7ff0000000000000LL;
   double w0, w1, w2;
-  if (t40 <= mn && t41 > mn) {
+  if (numbers && t40 <= mn && t41 > mn) {
     w0 = 1. / 3.; w1 = 2. / 3.; w2 = 0.;
-  } else if (t40 > mn && t41 < mn) {
+  } else if (numbers && t40 > mn && t41 < mn) {
     w0 = 0.; w1 = 2. / 3.; w2 = 1. / 3.;
   } else {
     const double eps = 1.E-2;

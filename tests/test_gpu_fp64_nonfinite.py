@@ -8,7 +8,7 @@ import pytest
 from conformal_cubed_sphere_gb300 import _lib as L
 from conformal_cubed_sphere_gb300 import model as M
 from oracle import oracle as O
-from tests.helpers import seeded_case
+from tests.helpers import CHECK_FIELDS, seeded_case
 
 pytestmark = pytest.mark.gpu
 
@@ -69,4 +69,34 @@ def test_doubled_tendencies_that_overflow(seed):
     g.step(1)
     a, b = g.get_state(), o.get_state(1)
     for k in ("phiG", "u", "v"):
+        _same(a[k], b[k], m, k)
+
+
+@pytest.mark.parametrize("seed", range(24))
+def test_damaged_states(seed):
+    """Cells set to zeros, infinities, NaNs, subnormals and magnitudes whose smoothness
+    indicators or products overflow: NaNs and infinities come out where the oracle has them
+    (a comparison of the WENO switches with a NaN is false)."""
+    rng = np.random.default_rng(seed)
+    N, halo = int(rng.choice([8, 20, 33])), int(rng.choice([3, 4]))
+    mesh = M.Mesh(N, halo, pole_inverse=N % 2 == 1)
+    s = M.initial_state(mesh, kind=L.CCS_IC_SEEDED, seed=seed, lmax_oro=8)
+    dt = M.cfl_dt(mesh, s, 0.4)
+    values = [0.0, -0.0, np.inf, -np.inf, np.nan, 5e-324, -1e-310, 1e60, -1e100, 1e154, -1e157, 1e200, 1e300]
+    for k in rng.choice(["phiG", "u", "v", "phi", "uC", "vC"], 1 + seed % 3, replace=False):
+        cells = np.flatnonzero(rng.random(mesh.ncell) < rng.choice([0.003, 0.1]))
+        s[k][cells] = rng.choice(values, size=cells.size) if seed % 2 else rng.choice(values)
+    ediss, scheme = int(rng.integers(0, 2)), str(rng.choice(["RK4", "RK3_TVD"]))
+    g = M.Stepper(mesh, dt, precision="fp64", scheme=scheme, e_dissipation=ediss)
+    g.set_variant(seed % 3)
+    g.set_state(s)
+    o = O.Oracle.from_mesh(mesh, e_dissipation=ediss)
+    o.set_state(s.arrays)
+    im, m = mesh.interior_mask(), ~mesh.corner_mask()
+    for q, (a, b) in enumerate(zip(g.spatial_operator(), o.spatial_operator())):
+        _same(a, b, im, q)
+    g.step(1)
+    o.run(dt, 1, scheme)
+    a, b = g.get_state(), o.get_state()
+    for k in CHECK_FIELDS:
         _same(a[k], b[k], m, k)
