@@ -245,10 +245,9 @@ __device__ __forceinline__ bool in_window(double x) {
 // tau41 < mn), the differences rounded as FP64 rounds them.  Single precision decides
 // them when both differences are further from mn than its error: the betas as floats
 // relative to the largest exponent, cut to 20 bits (error 2^-20, the largest in [1, 2)), so
-// tau - mn is off by less than 4e-6.  A warp with a closer call takes the FP64 differences.
-// lanes: the warp's lanes in this call (all of them make the same vote).
-__device__ __forceinline__ void switches(const F64Ops &f, unsigned lanes, double be0, double be1, double be2,
-                                         long long mn, bool &first, bool &last) {
+// tau - mn is off by less than 4e-6.  A lane with a closer call takes the FP64 differences.
+__device__ __forceinline__ void switches(const F64Ops &f, double be0, double be1, double be2, long long mn,
+                                         bool &first, bool &last) {
   const int h0 = __double2hiint(be0), h1 = __double2hiint(be1), h2 = __double2hiint(be2);
   const int base = (max(max(h0, h1), h2) & 0x7ff00000) - (127 << 20);
   const float f0 = __int_as_float(max(h0 - base, 0) << 3), f1 = __int_as_float(max(h1 - base, 0) << 3),
@@ -257,7 +256,7 @@ __device__ __forceinline__ void switches(const F64Ops &f, unsigned lanes, double
   const float d40 = fabsf(f0 - f1) - fm, d41 = fabsf(f1 - f2) - fm;
   first = d40 < 0.f && d41 > 0.f;
   last = d40 > 0.f && d41 < 0.f;
-  if (__any_sync(lanes, !(fminf(fabsf(d40), fabsf(d41)) > 1e-5f))) {
+  if (!(fminf(fabsf(d40), fabsf(d41)) > 1e-5f)) {
     const long long t40 = abs_bits(f.sub(be0, be1)), t41 = abs_bits(f.sub(be1, be2));
     first = t40 <= mn && t41 > mn;
     last = t40 > mn && t41 < mn;
@@ -280,10 +279,9 @@ __device__ __forceinline__ double times(double a, softfp::Unp w) {
 //   G[0..5] at the cell, arrays SG apart: Q/3, 7/6 Q, 11/6 Q, 5/6 Q, 1/3 Q, 3 Q
 //   ga at the cell: 13/12 (second difference centred there)^2, same orientation
 // (Q/6 and 1/6 Q are exact halves of Q/3 and 1/3 Q; multiplications by 2, 4 and 1/4 are
-// exact and fuse.)  The quotients run on the integer pipes (ccs_softfp.cuh).  lanes: the
-// warp's lanes that call it together.
-__device__ __forceinline__ double side(const F64Ops &f, unsigned lanes, const double *Q, int s, const double *G,
-                                       int SG, int gs, const double *ga, int as) {
+// exact and fuse.)  The quotients run on the integer pipes (ccs_softfp.cuh).
+__device__ __forceinline__ double side(const F64Ops &f, const double *Q, int s, const double *G, int SG, int gs,
+                                       const double *ga, int as) {
   const double q3 = G[5 * SG];
   const double b0 = f.add(fma(-4., Q[-s], Q[-2 * s]), q3);
   const double b1 = f.sub(Q[-s], Q[s]);
@@ -296,18 +294,17 @@ __device__ __forceinline__ double side(const F64Ops &f, unsigned lanes, const do
   if (__double_as_longlong(be1) < mn) mn = __double_as_longlong(be1);
   if (__double_as_longlong(be2) < mn) mn = __double_as_longlong(be2);
   bool first, last;  // the reference's two switches to fixed weights
-  switches(f, lanes, be0, be1, be2, mn, first, last);
+  switches(f, be0, be1, be2, mn, first, last);
   using namespace softfp;
   double w0 = first ? 1. / 3. : 0., w1 = 2. / 3., w2 = first ? 0. : 1. / 3.;
   const double s0 = f.add(f.sub(G[-2 * gs], G[SG - gs]), G[2 * SG]);
   const double s1 = f.add(fma(-0.5, G[-gs], G[3 * SG]), G[4 * SG + gs]);
   const double s2 = fma(-0.5, G[4 * SG + 2 * gs], f.add(G[0], G[3 * SG + gs]));
-  const unsigned weighted = __ballot_sync(lanes, !first && !last);
   if (!first && !last) {
     // eps + beta: beta itself from 2^48 on (eps is less than half its last place), which
     // is every beta of the fluxes and phitG
     double e0 = be0, e1 = be1, e2 = be2;
-    if (__any_sync(weighted, mn < 0x42f0000000000000LL)) {
+    if (mn < 0x42f0000000000000LL) {
       const double eps = 1.E-2;
       e0 = f.add(eps, be0); e1 = f.add(eps, be1); e2 = f.add(eps, be2);
     }
@@ -428,10 +425,10 @@ __device__ __forceinline__ void reconstruct(Smem<T> &S, const F64Ops &f, const d
   for (int t0 = tid & ~31; t0 < 2 * NF; t0 += NT) {
     const int t = t0 + (tid & 31), face = t >> 1, minus = t & 1;
     double val = 0.;
-    bool in = false;
-    int cell = 0, lcell = 0, st = 0, ls = 0;  // the cell in the halo'd tile and on its line's arrays
-    const double *z = nullptr, *G = nullptr, *A = nullptr;
     if (t < 2 * NF) {
+      bool in;
+      int cell, lcell, st, ls;  // the cell in the halo'd tile and on its line's arrays
+      const double *z, *G, *A;
       if (face < NFX) {
         const int lj = face / (TX + 1), ci = face % (TX + 1) + 2 + minus;
         in = lj < ny && ci - 2 - minus <= nx;
@@ -452,16 +449,14 @@ __device__ __forceinline__ void reconstruct(Smem<T> &S, const F64Ops &f, const d
         G = GY + (SAME ? cell : lcell);
         A = AY + (minus ? NLY : 0);
       }
-      in = in && ccs_inb(cell - 2 * st, RN, 211) && ccs_inb(cell + 2 * st, RN, 212);
-    }
-    const unsigned lanes = __ballot_sync(0xffffffffu, in);  // (t0 is the warp's)
-    if (in) {
-      z += cell;
-      if (minus) { st = -st; ls = -ls; }
-      if (slow)
-        val = weno5z(z[-2 * st], z[-st], z[0], z[st], z[2 * st]);
-      else
-        val = side(f, lanes, z, st, G, face < NFX ? SGX : SGY, SAME ? st : ls, A + lcell, ls);
+      if (in && ccs_inb(cell - 2 * st, RN, 211) && ccs_inb(cell + 2 * st, RN, 212)) {
+        z += cell;
+        if (minus) { st = -st; ls = -ls; }
+        if (slow)
+          val = weno5z(z[-2 * st], z[-st], z[0], z[st], z[2 * st]);
+        else
+          val = side(f, z, st, G, face < NFX ? SGX : SGY, SAME ? st : ls, A + lcell, ls);
+      }
     }
     if (t0 + NT < 2 * NF && first_face < 0) {
       first = val;
@@ -808,7 +803,7 @@ __global__ void side_check_kernel(const double *__restrict__ a, int64_t n, F64Op
     for (int q = 0; q < 5; q++) Q[q] = a[5 * w + q];
     for (int q = 0; q < 5; q++) store_singles(f, G + q, 5, Q[q]);
     for (int q = 0; q < 3; q++) ga[q] = curvature(f.add(fma(-2., Q[q + 1], Q[q]), Q[q + 2]));
-    const double fast = side(f, 0xffffffffu, Q + 2, 1, G + 2, 5, 1, ga + 1, 1);
+    const double fast = side(f, Q + 2, 1, G + 2, 5, 1, ga + 1, 1);
     const double ieee = weno5z(Q[0], Q[1], Q[2], Q[3], Q[4]);
     if (k < m) {
       out[k] = fast;
