@@ -222,13 +222,12 @@ __device__ __forceinline__ double half_of(double x) {
   return 0.5 * x;
 }
 
-// 2 x by its exponent; zeros, subnormals, infinities, NaNs and values whose double
-// overflows take the FP64 multiplication.  (fma(2, x, a) would not overflow where the
-// reference's 2 x does.)
-__device__ __forceinline__ double twice(double x) {
-  const uint32_t h = softfp::hi32(softfp::bits_of(x)), e = h & 0x7ff00000u;
-  if (e - 0x00100000u < 0x7fd00000u) return __hiloint2double((int)(h + 0x00100000u), __double2loint(x));
-  return 2. * x;
+// x as RK4's doubled tendencies take it: where 2 x overflows an infinity, so that
+// fma(2, x, a) is infinite where the reference's a + 2 x is
+__device__ __forceinline__ double to_double(double x) {
+  const uint32_t h = softfp::hi32(softfp::bits_of(x));
+  const bool over = (h & 0x7ff00000u) == 0x7fe00000u;
+  return __hiloint2double((int)(over ? (h & 0x80000000u) | 0x7ff00000u : h), over ? 0 : __double2loint(x));
 }
 
 // Whether the integer arithmetic of the reconstructions covers a field value: zero or
@@ -676,7 +675,7 @@ f64_stage_kernel(const F64Stage *__restrict__ stages, const WorkItem *__restrict
           double n[3];
           if (kind == K_RK4_2)
 #pragma unroll
-            for (int q = 0; q < 3; q++) ac[q] = f.add(ac[q], twice(t[q]));
+            for (int q = 0; q < 3; q++) ac[q] = fma(2., to_double(t[q]), ac[q]);
 #pragma unroll
           for (int q = 0; q < 3; q++) {
             if (kind == K_RK4_4)
