@@ -131,6 +131,14 @@ constexpr int MX_NVAR = 4;  // 32 x 32 (256 threads), 32 x 16 (128 threads); eac
 constexpr TileShape kMxTiles[MX_NVAR] = {{32, 32}, {32, 16}, {32, 32}, {32, 16}};
 constexpr int kMxStaging[MX_NVAR] = {kStageLoads, kStageLoads, kStageAsync, kStageAsync};
 
+// Whether a launch of nwork whole mixed tiles on sms SMs may be chained.  With at most two
+// 32 x 32 tiles an SM, every SM has room for a third: CTAs that start early crowd onto the
+// SMs that drain first, and a stage takes as long as an SM with three (us a step, four steps a
+// call, chained / not: C193 66.2 / 60.0, C208 63.8 / 60.1, C224 64.2 / 60.0; with more than two
+// C240 72.8 / 75.9, C256 74.1 / 76.4).  32 x 16 tiles, five an SM, are faster chained but for
+// the fullest rounds (C200 56.0 / 58.0, C224 62.7 / 62.0).
+constexpr bool mixed_chains(TileShape tile, int nwork, int sms) { return tile.ty != 32 || nwork > 2 * sms; }
+
 // kernel launchers (return cudaGetLastError()); `var` indexes the tile tables
 // (central: every stage in d_stages uses a central-difference operator, else WENO-Z)
 cudaError_t launch_f64_stage(int var, bool central, const F64Stage *d_stages, const WorkItem *d_work, int nwork,

@@ -1008,7 +1008,11 @@ int mixed_max_grid(int var, int device) {
 // operands in flight before the wait: C24 4.6, C48 5.1, C96 6.7, C128 9.3, C192 12.8)
 // Same bits in every tile shape.
 enum { kWhole, kMid, kSmall };
-static cudaError_t mixed_parts(int var, int nwork, int *size) {
+static cudaError_t mixed_parts(int var, int nwork, int *size, int *sms) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e == cudaSuccess) e = cudaDeviceGetAttribute(sms, cudaDevAttrMultiProcessorCount, dev);
+  if (e != cudaSuccess) return e;
   const TileShape ts = kMxTiles[var];
   const int small = nwork * (ts.tx / MxS::TX) * (ts.ty / MxS::TY), mid = nwork * (ts.tx / MxM::TX) * (ts.ty / MxM::TY);
 #ifdef CCS_BOUNDS
@@ -1017,11 +1021,7 @@ static cudaError_t mixed_parts(int var, int nwork, int *size) {
   // or 12 (48 small parts either way)
   const int most_small = 48, most_mid = 72;
 #else
-  int dev = 0, sms = 0;
-  cudaError_t e = cudaGetDevice(&dev);
-  if (e == cudaSuccess) e = cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
-  if (e != cudaSuccess) return e;
-  const int most_small = 3 * sms, most_mid = 6 * sms;
+  const int most_small = 3 * *sms, most_mid = 6 * *sms;
 #endif
   *size = small <= most_small ? kSmall : mid <= most_mid ? kMid : kWhole;
   return cudaSuccess;
@@ -1030,8 +1030,8 @@ static cudaError_t mixed_parts(int var, int nwork, int *size) {
 cudaError_t launch_mixed_stage(int var, bool central, bool ediss, const MixedStage *d_stages,
                                const WorkItem *d_work, int nwork, int grid, cudaStream_t s,
                                bool chained) {
-  int size = kWhole;
-  const cudaError_t e = mixed_parts(var, nwork, &size);
+  int size = kWhole, sms = 0;
+  const cudaError_t e = mixed_parts(var, nwork, &size, &sms);
   if (e != cudaSuccess) return e;
   const TileShape ts = kMxTiles[var];
   if (size == kSmall) {
@@ -1042,6 +1042,7 @@ cudaError_t launch_mixed_stage(int var, bool central, bool ediss, const MixedSta
     const int sx = ts.tx / MxM::TX, sy = ts.ty / MxM::TY;
     return mx_launch_any<MxM, kStageLoads>(central, ediss, d_stages, d_work, nwork, sx, sy, nwork * sx * sy, s, chained);
   }
+  chained = chained && mixed_chains(ts, nwork, sms);
   switch (var) {
     case 1: return mx_launch_any<MxT1, kStageLoads>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s, chained);
     case 2: return mx_launch_any<MxT0, kStageAsync>(central, ediss, d_stages, d_work, nwork, 1, 1, grid, s, chained);
@@ -1051,8 +1052,8 @@ cudaError_t launch_mixed_stage(int var, bool central, bool ediss, const MixedSta
 }
 
 cudaError_t mixed_stage_tile(int var, int nwork, StageTile *tile) {
-  int size = kWhole;
-  const cudaError_t e = mixed_parts(var, nwork, &size);
+  int size = kWhole, sms = 0;
+  const cudaError_t e = mixed_parts(var, nwork, &size, &sms);
   if (e != cudaSuccess) return e;
   if (size != kWhole)
     *tile = size == kSmall ? mx_tile_of<MxS, kStageAsync>() : mx_tile_of<MxM, kStageLoads>();
