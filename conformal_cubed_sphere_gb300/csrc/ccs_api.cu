@@ -172,8 +172,9 @@ static const int kDiagBlocks = 512;
 
 // Steps of the graph that a run of many steps replays: consecutive graphs leave the GPU
 // idle for about 4 us, as long as a stage of a small grid (mixed C48 6.2 -> 5.1 us a stage,
-// C96 7.7 -> 6.7, C384 33.4 -> 32.7; FP64 C48 29.5 -> 28.6).  Captured when a call asks for
-// at least twice as many steps, so that short calls do not pay for the larger graph.
+// C96 7.7 -> 6.7, C384 33.4 -> 32.7; FP64 C48 29.5 -> 28.6).  Captured when a call runs at
+// least twice as many (16 steps; on the FP64 lane and in batches, whose last step is a graph
+// of its own, 17), so that short calls do not pay for the larger graph.
 constexpr int kGraphSteps = 8;
 
 // Copies n fields of `bytes` each (dst[q] <- src[q], NULL entries skipped), one
@@ -1352,10 +1353,10 @@ static int set_variant(ccs_handle *h, int var) {
 }
 
 // Mean time of one stage launch with the handle's current variant, over the RK
-// stages before the last one, in step order and chained as a step's stages are.  Those stages read the state and
-// write only stage scratch (the next stage's input and the RK accumulator); the
-// last stage, which writes the state, is the only one left out, so timing leaves
-// the state unchanged.
+// stages before the last one, in step order and chained as a step's stages are.  Those
+// stages read the state and write only stage scratch (the next stage's input and the RK
+// accumulator); the last stage, which writes the state, is the only one left out, so
+// timing leaves the state unchanged.
 static int time_stages(ccs_handle *h, int reps, double *us) {
   const bool mx = h->cfg.precision == CCS_MIXED;
   const int nst = (mx ? h->mixed->n_rk : h->n_rk) - 1;
@@ -1549,8 +1550,9 @@ static int group_set_var(ccs_batch *b, BatchGroup &g, int var) {
 }
 
 // n steps of every group (with_sw: the last one with the sphere winds): the groups fork
-// from the batch stream, run their RK stages on their own streams (an FP64 group is FP64-issue bound and a mixed group
-// FP32 / latency bound, so they share the SMs well) and join back.
+// from the batch stream, run their RK stages on their own streams and join back (an SM
+// with two FP64 CTAs has no registers left for a mixed one, so the mixed stages mostly run
+// in the FP64 stages' tails).
 static int batch_enqueue(ccs_batch *b, int n, bool with_sw) {
   BATCH_TRY(b, cudaEventRecord(b->fork, b->stream));
   for (auto &g : b->groups) {

@@ -754,7 +754,7 @@ mixed_stage_kernel(const MixedStage *__restrict__ stages, const WorkItem *__rest
       for (int k = tid; k < nwd; k += NT) cp_async4(reinterpret_cast<float *>(dst + k),
                                                       reinterpret_cast<const float *>(src + k));
     }
-    // ---- phase 2: lines -> face values (warps 0-3 rows, 4-7 columns) ---------
+    // ---- phase 2: lines -> face values (the first NTX threads rows, the others columns) ----
     if (!CENTRAL) {  // (the central-difference operators have no faces)
       // segment seg of a line covers faces 0 .. SEG (seg 0) or SEG seg + 1 .. SEG seg + SEG
       if (tid < T::NTX) {
